@@ -89,7 +89,7 @@ struct gvx_batch {
   std::vector<gvx_dvm*> maps;
   gvx::BatchMap* d_table = nullptr;
   gvx::BatchItems items{};
-  long long* d_prefix = nullptr;  // 3 x (n_maps + 1)
+  long long* d_prefix = nullptr;  // 6 x (n_maps + 1)
   uint32_t* d_stacks = nullptr;   // fused Y -> X: one stack per resident warp
   unsigned* d_sync = nullptr;     // slice counters of all maps, queue head, error word
   cudaGraph_t graph = nullptr;
@@ -105,7 +105,8 @@ gvx_status gvx_batch_create(gvx_dvm* const* maps, uint32_t n_maps, gvx_batch** o
   if (out == nullptr || maps == nullptr || n_maps == 0) return fail(GVX_ERR_INVALID_ARG, "need at least one map");
   *out = nullptr;
   std::vector<BatchMap> table(n_maps);
-  uint32_t sync_words = 0, stack_len = 1, z_max = 1;
+  uint32_t sync_words = 0, stack_len = 1, x_max = 1, y_max = 1, z_max = 1;
+  bool search = true;
   for (uint32_t k = 0; k < n_maps; ++k) {
     if (maps[k] == nullptr) return fail(GVX_ERR_INVALID_ARG, "null map in batch");
     const gvx_dvm* m = maps[k];
@@ -113,19 +114,23 @@ gvx_status gvx_batch_create(gvx_dvm* const* maps, uint32_t n_maps, gvx_batch** o
                         (int)m->dims.z, m->side, num_voxels(m->dims), sync_words};
     sync_words += m->dims.z;
     stack_len = std::max(stack_len, std::max(m->dims.x, m->dims.y));
+    x_max = std::max(x_max, m->dims.x);
+    y_max = std::max(y_max, m->dims.y);
     z_max = std::max(z_max, m->dims.z);
+    search = search && search_takes(m->dims);
   }
   const long long stack_warps = edt_batch_stack_warps();
   if (stack_warps <= 0) return fail(GVX_ERR_CUDA, "occupancy query for the batched EDT failed");
   gvx_batch* b = new (std::nothrow) gvx_batch();
   if (b == nullptr) return fail(GVX_ERR_OOM, "host allocation failed");
   b->maps.assign(maps, maps + n_maps);
-  std::vector<long long> prefix(4 * (size_t)(n_maps + 1), 0);
-  for (int p = 0; p < 4; ++p) {
+  std::vector<long long> prefix(6 * (size_t)(n_maps + 1), 0);
+  for (int p = 0; p < 6; ++p) {
     for (uint32_t k = 0; k < n_maps; ++k) {
       const gvx_dims& d = maps[k]->dims;
-      const long long items = p < 3 ? edt_pass_items(d, p)  // occupancy tasks: z items x 32-row chunks
-                                    : edt_pass_items(d, 0) * (long long)((d.z + 31) / 32);
+      const long long items = p < 3 ? edt_pass_items(d, p)
+                              : p == 3 ? edt_pass_items(d, 0) * (long long)((d.z + 31) / 32)  // z items x 32-row chunks
+                                       : search_items(d, p - 3);
       prefix[p * (n_maps + 1) + k + 1] = prefix[p * (n_maps + 1) + k] + items;
     }
     b->items.total[p] = prefix[p * (n_maps + 1) + n_maps];
@@ -146,13 +151,16 @@ gvx_status gvx_batch_create(gvx_dvm* const* maps, uint32_t n_maps, gvx_batch** o
     delete b;
     return cuda_status(e, "batch table");
   }
-  for (int p = 0; p < 4; ++p) b->items.d_prefix[p] = b->d_prefix + p * (size_t)(n_maps + 1);
+  for (int p = 0; p < 6; ++p) b->items.d_prefix[p] = b->d_prefix + p * (size_t)(n_maps + 1);
   b->items.d_stacks = b->d_stacks;
   b->items.stack_warps = stack_warps;
   b->items.stack_len = stack_len;
   b->items.d_sync = b->d_sync;
   b->items.sync_words = sync_words;
+  b->items.x_max = x_max;
+  b->items.y_max = y_max;
   b->items.z_max = z_max;
+  b->items.search = search && b->items.total[4] < (1ll << 31) && b->items.total[5] < (1ll << 31);
   *out = b;
   return GVX_OK;
 }

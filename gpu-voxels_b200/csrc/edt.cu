@@ -5,6 +5,12 @@
 // nearest site, including the reference's tie-breaking -- for any dims in
 // [1,1023]^3 (the reference itself needs x == y and x % 64 == 0).
 //
+// Maps whose sites all lie in their own voxels (after insertPointCloud, or
+// voxelize_edt's occupancy bits) and whose rows and columns have at most 512
+// voxels go to the row search (edt_search.cu).  The sweeps below take the
+// others: longer axes, maps transformed before or written by the caller, the
+// workspace built into the library, and the single-stage entry point.
+//
 // Three sweeps (pass Z one launch, passes Y and X one fused launch):
 //   pass Z : phase 1 (kernelPBAphase1FloodZ, VoxelMapOperationsPBA.hpp:63-124)
 //            per (x,y) column.
@@ -78,10 +84,6 @@ constexpr int kZWarps = 8;
 __host__ __device__ constexpr int z_bits_words(int Z) { return 32 * ((Z + 31) >> 5); }
 constexpr int kZBitsSmemMax = kZWarps * 2 * z_bits_words(1024) * 4;
 constexpr int kZWarpWords = 2 * kZChunk * 32 + 2 * kZRing * 32;
-
-// Words of the EDT workspace's counter area (Z slice counters, queue head,
-// error word, pass Z's other-sites flag, padded to 32).
-__host__ __device__ __forceinline__ uint64_t edt_sync_words(int Z) { return ((uint64_t)Z + 3 + 31) / 32 * 32; }
 
 // Workspace words of pass Z's chunk carries for a map: per warp item
 // (32 columns) one word per lane and chunk.
@@ -923,6 +925,13 @@ __device__ __forceinline__ void sweep_item(uint32_t* __restrict__ map, uint32_t*
 // A map's other-sites flag in a batch: word Z + 2 of its workspace, as for one map.
 __device__ __forceinline__ uint32_t* batch_other(const BatchMap& m) { return m.scratch + m.Z + 2; }
 
+// Whether any map of the batch has its other-sites flag set (all threads call).
+__device__ __forceinline__ bool any_other(const BatchMap* __restrict__ maps, uint32_t n_maps) {
+  int any = 0;
+  for (uint32_t k = threadIdx.x; k < n_maps; k += blockDim.x) any |= *batch_other(maps[k]) != 0u;
+  return __syncthreads_or(any) != 0;
+}
+
 // Map owning warp item g of a batch pass: last k with prefix[k] <= g.
 __device__ __forceinline__ uint32_t batch_owner(const long long* __restrict__ prefix, uint32_t n, long long g) {
   uint32_t lo = 0, hi = n;
@@ -951,6 +960,7 @@ __global__ void __launch_bounds__(kZWarps * 32, 3) edt_pass_z_batch(const BatchM
                                                                      const long long* __restrict__ prefix,
                                                                      uint32_t n_maps, long long total) {
   extern __shared__ __align__(16) uint32_t s_z[];
+  if (!any_other(maps, n_maps)) return;
   const int warp = threadIdx.x >> 5;
   for (long long g = (long long)blockIdx.x * kZWarps + warp; g < total; g += (long long)gridDim.x * kZWarps) {
     const uint32_t k = batch_owner(prefix, n_maps, g);
@@ -1138,9 +1148,11 @@ __global__ void __launch_bounds__(kZWarps * 32) edt_pass_z_bits_batch(const Batc
 // schedule below): persistent warps stride over the items, one stack each.
 template <bool kXPass, int kRows>
 __global__ void __launch_bounds__(SweepCfg<kRows>::kWarps * 32, 3)
-    edt_sweep(uint32_t* __restrict__ map, uint32_t* __restrict__ stacks, int X, int Y, int Z) {
+    edt_sweep(uint32_t* __restrict__ map, uint32_t* __restrict__ stacks, int X, int Y, int Z,
+              const uint32_t* __restrict__ run_if) {
   using Cfg = SweepCfg<kRows>;
   extern __shared__ __align__(16) uint32_t s_sweep[];  // [kWarps][kWarpWords]
+  if (run_if != nullptr && *run_if == 0u) return;
   const int warp = threadIdx.x >> 5;
   const long long gw = (long long)blockIdx.x * Cfg::kWarps + warp;
   uint32_t* stack = stacks + (uint64_t)gw * warp_stack_words(X, Y);
@@ -1234,9 +1246,10 @@ __device__ __forceinline__ unsigned next_item(unsigned* head) {
 template <int kRows>
 __global__ void __launch_bounds__(SweepCfg<kRows>::kWarps * 32, 3)
     edt_sweep_yx(uint32_t* __restrict__ map, uint32_t* __restrict__ stacks, unsigned* __restrict__ sync, int X, int Y,
-                 int Z) {
+                 int Z, const uint32_t* __restrict__ run_if) {
   using Cfg = SweepCfg<kRows>;
   extern __shared__ __align__(16) uint32_t s_sweep[];
+  if (run_if != nullptr && *run_if == 0u) return;
   const int warp = threadIdx.x >> 5;
   uint32_t* wbase = s_sweep + (size_t)warp * Cfg::kWarpWords;
   uint32_t* stack = stacks + ((uint64_t)blockIdx.x * Cfg::kWarps + warp) * warp_stack_words(X, Y);
@@ -1268,15 +1281,16 @@ __global__ void __launch_bounds__(SweepCfg<kRows>::kWarps * 32, 3)
 // items, then all maps' X items.  maps[k].sync_off locates map k's slice
 // counters in `sync`; the queue head and error word follow them.  Both passes
 // of a map whose pass Z took the occupancy-bit route (its other-sites flag
-// clear) run sweep_item's kOwnA form.
+// clear) run sweep_item's kOwnA form; others_only: those maps are left out.
 template <int kRows>
 __global__ void __launch_bounds__(SweepCfg<kRows>::kWarps * 32, 3)
     edt_sweep_yx_batch(const BatchMap* __restrict__ maps, const long long* __restrict__ prefix_y,
                        const long long* __restrict__ prefix_x, uint32_t n_maps, unsigned total_y, unsigned total_x,
                        uint32_t* __restrict__ stacks, uint32_t stack_len, unsigned* __restrict__ sync,
-                       unsigned sync_words) {
+                       unsigned sync_words, int others_only) {
   using Cfg = SweepCfg<kRows>;
   extern __shared__ __align__(16) uint32_t s_sweep[];
+  if (others_only && !any_other(maps, n_maps)) return;
   const int warp = threadIdx.x >> 5;
   uint32_t* wbase = s_sweep + (size_t)warp * Cfg::kWarpWords;
   uint32_t* stack = stacks + ((uint64_t)blockIdx.x * Cfg::kWarps + warp) * (uint64_t)stack_len * 64;
@@ -1292,6 +1306,7 @@ __global__ void __launch_bounds__(SweepCfg<kRows>::kWarps * 32, 3)
     const unsigned item = (unsigned)(q - __ldg(prefix + k));
     unsigned* done = sync + m.sync_off;
     unsigned za, zb;
+    if (others_only && *batch_other(m) == 0u) continue;  // the row search took this map
     if (!x_item) {
       if (*batch_other(m) == 0u) sweep_item<false, kRows, true>(m.vox, stack, m.X, m.Y, m.Z, item, wbase);
       else sweep_item<false, kRows, false>(m.vox, stack, m.X, m.Y, m.Z, item, wbase);
@@ -1353,6 +1368,17 @@ cudaError_t kernel_setup(int threads, int smem, long long* resident) {
   return st.err[dev];
 }
 
+// The general pass Z, run only when the other-sites flag is set.
+cudaError_t launch_pass_z_general(uint32_t* map, uint32_t* scratch, gvx_dims d, cudaStream_t s) {
+  const int smem = kZWarps * kZWarpWords * 4;
+  cudaError_t e = kernel_setup<edt_pass_z>(kZWarps * 32, smem, nullptr);
+  if (e != cudaSuccess) return e;
+  const unsigned blocks = (unsigned)((z_items((int)d.x, (int)d.y) + kZWarps - 1) / kZWarps);
+  edt_pass_z<<<blocks, kZWarps * 32, smem, s>>>(map, scratch + edt_sync_words((int)d.z), (int)d.x, (int)d.y, (int)d.z,
+                                                scratch + (uint64_t)d.z + 2);
+  return cudaGetLastError();
+}
+
 // Pass Z of a filled map: occupancy bits from the map, then the bits pass;
 // when some voxel holds another site than its own, the bits pass skips and
 // the general pass runs (both are launched; the flag picks on the device).
@@ -1380,10 +1406,7 @@ cudaError_t launch_pass_z(uint32_t* map, uint32_t* scratch, gvx_dims d, cudaStre
   if ((e = kernel_setup<edt_pass_z_bits>(kZWarps * 32, kZBitsSmemMax, nullptr)) != cudaSuccess) return e;
   edt_pass_z_bits<<<z_blocks, kZWarps * 32, kZWarps * 2 * z_bits_words(Z) * 4, s>>>(map, area, X, Y, Z, other);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  const int smem = kZWarps * kZWarpWords * 4;
-  if ((e = kernel_setup<edt_pass_z>(kZWarps * 32, smem, nullptr)) != cudaSuccess) return e;
-  edt_pass_z<<<z_blocks, kZWarps * 32, smem, s>>>(map, area, X, Y, Z, other);
-  return cudaGetLastError();
+  return launch_pass_z_general(map, scratch, d, s);
 }
 
 // Workspace layout: [slice counters, queue head, error word: sync_words(d)]
@@ -1400,7 +1423,8 @@ long long sweep_blocks(long long resident, uint64_t stack_area, gvx_dims d, int 
 }
 
 template <bool kXPass, int kRows>
-cudaError_t launch_sweep(uint32_t* map, uint32_t* scratch, uint64_t scratch_words, gvx_dims d, cudaStream_t s) {
+cudaError_t launch_sweep(uint32_t* map, uint32_t* scratch, uint64_t scratch_words, gvx_dims d, cudaStream_t s,
+                         const uint32_t* run_if) {
   using Cfg = SweepCfg<kRows>;
   const long long items = edt_pass_items(d, kXPass ? 2 : 1);
   const int smem = Cfg::kWarps * Cfg::kWarpWords * 4;
@@ -1410,7 +1434,7 @@ cudaError_t launch_sweep(uint32_t* map, uint32_t* scratch, uint64_t scratch_word
   blocks = sweep_blocks(blocks, scratch_words - sync_words(d), d, Cfg::kWarps, items);
   if (blocks < 1) return cudaErrorInvalidValue;
   edt_sweep<kXPass, kRows><<<(unsigned)blocks, Cfg::kWarps * 32, smem, s>>>(map, scratch + sync_words(d), (int)d.x,
-                                                                             (int)d.y, (int)d.z);
+                                                                             (int)d.y, (int)d.z, run_if);
   return cudaGetLastError();
 }
 
@@ -1426,7 +1450,8 @@ uint64_t fused_stack_words(gvx_dims d) {
 // Fused Y -> X launch for one map: as many blocks as are resident, as the
 // stack area holds and as there are items.
 template <int kRows>
-cudaError_t launch_sweep_yx(uint32_t* map, uint32_t* scratch, uint64_t scratch_words, gvx_dims d, cudaStream_t s) {
+cudaError_t launch_sweep_yx(uint32_t* map, uint32_t* scratch, uint64_t scratch_words, gvx_dims d, cudaStream_t s,
+                            const uint32_t* run_if) {
   using Cfg = SweepCfg<kRows>;
   const int smem = Cfg::kWarps * Cfg::kWarpWords * 4;
   long long blocks = 0;
@@ -1439,7 +1464,7 @@ cudaError_t launch_sweep_yx(uint32_t* map, uint32_t* scratch, uint64_t scratch_w
   e = cudaMemsetAsync(sync, 0, (d.z + 2) * sizeof(unsigned), s);
   if (e != cudaSuccess) return e;
   edt_sweep_yx<kRows><<<(unsigned)blocks, Cfg::kWarps * 32, smem, s>>>(map, scratch + sync_words(d), sync, (int)d.x,
-                                                                       (int)d.y, (int)d.z);
+                                                                       (int)d.y, (int)d.z, run_if);
   return cudaGetLastError();
 }
 
@@ -1456,7 +1481,7 @@ int sweep_rows() {
 }
 
 template <int kRows>
-cudaError_t launch_yx_batch(const BatchMap* d_table, const BatchItems& it, cudaStream_t s) {
+cudaError_t launch_yx_batch(const BatchMap* d_table, const BatchItems& it, cudaStream_t s, int others_only) {
   using Cfg = SweepCfg<kRows>;
   const int smem = Cfg::kWarps * Cfg::kWarpWords * 4;
   auto kern = edt_sweep_yx_batch<kRows>;
@@ -1470,7 +1495,7 @@ cudaError_t launch_yx_batch(const BatchMap* d_table, const BatchItems& it, cudaS
   if (e != cudaSuccess) return e;
   kern<<<(unsigned)blocks, Cfg::kWarps * 32, smem, s>>>(d_table, it.d_prefix[1], it.d_prefix[2], it.n_maps,
                                                         (unsigned)it.total[1], (unsigned)it.total[2], it.d_stacks,
-                                                        it.stack_len, it.d_sync, it.sync_words);
+                                                        it.stack_len, it.d_sync, it.sync_words, others_only);
   return cudaGetLastError();
 }
 
@@ -1512,34 +1537,68 @@ uint64_t edt_scratch_words_min(gvx_dims d) {
                                              zcarry_words(d), occ_words((int)d.x, (int)d.y, (int)d.z)});
 }
 uint64_t edt_scratch_words(gvx_dims d) {
-  return std::max(sync_words(d) + fused_stack_words(d), edt_scratch_words_min(d));
+  const uint64_t sweeps = std::max(sync_words(d) + fused_stack_words(d), edt_scratch_words_min(d));
+  return search_takes(d) ? std::max(sweeps, sync_words(d) + search_words(d)) : sweeps;
 }
+
+namespace {
+
+// One sweep launch (pass 1 = Y, 2 = X, 3 = fused Y -> X); run_if (optional):
+// only when this flag is set.
+cudaError_t launch_sweep_pass(uint32_t* d_vox, uint32_t* d_scratch, uint64_t scratch_words, gvx_dims d, int pass,
+                              cudaStream_t s, int rows, const uint32_t* run_if) {
+  const bool big = (rows == 0 ? sweep_rows() : rows) == 32;
+  switch (pass) {
+    case 1:
+      return big ? launch_sweep<false, 32>(d_vox, d_scratch, scratch_words, d, s, run_if)
+                 : launch_sweep<false, 16>(d_vox, d_scratch, scratch_words, d, s, run_if);
+    case 2:
+      return big ? launch_sweep<true, 32>(d_vox, d_scratch, scratch_words, d, s, run_if)
+                 : launch_sweep<true, 16>(d_vox, d_scratch, scratch_words, d, s, run_if);
+    default:
+      return big ? launch_sweep_yx<32>(d_vox, d_scratch, scratch_words, d, s, run_if)
+                 : launch_sweep_yx<16>(d_vox, d_scratch, scratch_words, d, s, run_if);
+  }
+}
+
+// The sweeps after pass Z, fused or one by one.
+cudaError_t launch_sweeps(uint32_t* d_vox, uint32_t* d_scratch, uint64_t scratch_words, gvx_dims d, cudaStream_t s,
+                          const EdtConfig& cfg, const uint32_t* run_if) {
+  if (cfg.fused) return launch_sweep_pass(d_vox, d_scratch, scratch_words, d, 3, s, cfg.rows, run_if);
+  const cudaError_t e = launch_sweep_pass(d_vox, d_scratch, scratch_words, d, 1, s, cfg.rows, run_if);
+  return e == cudaSuccess ? launch_sweep_pass(d_vox, d_scratch, scratch_words, d, 2, s, cfg.rows, run_if) : e;
+}
+
+// Whether the row search (edt_search.cu) takes maps of these dims in this
+// workspace (a map handle's always holds it; the built-in one is too small for
+// some maps that the sweeps fit in).
+bool use_search(gvx_dims d, uint64_t scratch_words) {
+  return search_takes(d) && scratch_words >= sync_words(d) + search_words(d);
+}
+
+}  // namespace
 
 cudaError_t launch_edt_pass(uint32_t* d_vox, uint32_t* d_scratch, uint64_t scratch_words, gvx_dims d, int pass,
                             cudaStream_t s, int rows) {
-  if (scratch_words < edt_scratch_words_min(d)) return cudaErrorInvalidValue;
-  const bool big = (rows == 0 ? sweep_rows() : rows) == 32;
-  switch (pass) {
-    case 0: return launch_pass_z(d_vox, d_scratch, d, s);
-    case 1:
-      return big ? launch_sweep<false, 32>(d_vox, d_scratch, scratch_words, d, s)
-                 : launch_sweep<false, 16>(d_vox, d_scratch, scratch_words, d, s);
-    case 2:
-      return big ? launch_sweep<true, 32>(d_vox, d_scratch, scratch_words, d, s)
-                 : launch_sweep<true, 16>(d_vox, d_scratch, scratch_words, d, s);
-    case 3:
-      return big ? launch_sweep_yx<32>(d_vox, d_scratch, scratch_words, d, s)
-                 : launch_sweep_yx<16>(d_vox, d_scratch, scratch_words, d, s);
-    default: return cudaErrorInvalidValue;
-  }
+  if (scratch_words < edt_scratch_words_min(d) || pass < 0 || pass > 3) return cudaErrorInvalidValue;
+  if (pass == 0) return launch_pass_z(d_vox, d_scratch, d, s);
+  return launch_sweep_pass(d_vox, d_scratch, scratch_words, d, pass, s, rows, nullptr);
 }
 
 cudaError_t launch_edt(uint32_t* d_vox, uint32_t* d_scratch, uint64_t scratch_words, gvx_dims d, cudaStream_t s,
                        const EdtConfig& cfg) {
-  cudaError_t e = launch_edt_pass(d_vox, d_scratch, scratch_words, d, 0, s, cfg.rows);
-  if (e != cudaSuccess || cfg.fused) return e == cudaSuccess ? launch_edt_pass(d_vox, d_scratch, scratch_words, d, 3, s, cfg.rows) : e;
-  e = launch_edt_pass(d_vox, d_scratch, scratch_words, d, 1, s, cfg.rows);
-  return e == cudaSuccess ? launch_edt_pass(d_vox, d_scratch, scratch_words, d, 2, s, cfg.rows) : e;
+  if (scratch_words < edt_scratch_words_min(d)) return cudaErrorInvalidValue;
+  if (!use_search(d, scratch_words)) {
+    const cudaError_t e = launch_pass_z(d_vox, d_scratch, d, s);
+    return e == cudaSuccess ? launch_sweeps(d_vox, d_scratch, scratch_words, d, s, cfg, nullptr) : e;
+  }
+  // The row search takes a map whose sites are all their own voxels; the flag
+  // it sets otherwise lets the general pass Z and the sweeps run.
+  uint32_t* other = d_scratch + (uint64_t)d.z + 2;
+  cudaError_t e = cudaMemsetAsync(d_scratch, 0, ((uint64_t)d.z + 3) * sizeof(uint32_t), s);
+  if (e == cudaSuccess) e = launch_search_filled(d_vox, d_scratch + sync_words(d), d, other, s);
+  if (e == cudaSuccess) e = launch_pass_z_general(d_vox, d_scratch, d, s);
+  return e == cudaSuccess ? launch_sweeps(d_vox, d_scratch, scratch_words, d, s, cfg, other) : e;
 }
 
 cudaError_t edt_read_error(const uint32_t* d_scratch, gvx_dims d, uint32_t* flag) {
@@ -1562,6 +1621,12 @@ cudaError_t launch_voxelize_edt(uint32_t* d_vox, uint32_t* d_scratch, uint64_t s
                                 const float* d_xyz, uint64_t n, uint32_t* d_outside, cudaStream_t s,
                                 const EdtConfig& cfg) {
   if (scratch_words < edt_scratch_words_min(d)) return cudaErrorInvalidValue;
+  if (use_search(d, scratch_words)) {  // the error word and the occupancy bits in one memset
+    uint32_t* err = d_scratch + (uint64_t)d.z + 1;
+    uint32_t* area = d_scratch + sync_words(d);
+    const cudaError_t e = cudaMemsetAsync(err, 0, (area - err + search_bits_words(d)) * sizeof(uint32_t), s);
+    return e == cudaSuccess ? launch_search_voxelize(d_vox, area, d, side, d_xyz, n, d_outside, s) : e;
+  }
   uint32_t* bits = d_scratch + edt_sync_words((int)d.z);
   // the occupancy bits and, in the same memset, pass Z's other-sites flag
   // (every site is its own: the fused sweep's pass Y may skip the x offset)
@@ -1580,9 +1645,7 @@ cudaError_t launch_voxelize_edt(uint32_t* d_vox, uint32_t* d_scratch, uint64_t s
   edt_pass_z_bits<<<(unsigned)((items + kZWarps - 1) / kZWarps), kZWarps * 32, smem, s>>>(d_vox, bits, (int)d.x,
                                                                                          (int)d.y, (int)d.z, nullptr);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if (cfg.fused) return launch_edt_pass(d_vox, d_scratch, scratch_words, d, 3, s, cfg.rows);
-  e = launch_edt_pass(d_vox, d_scratch, scratch_words, d, 1, s, cfg.rows);
-  return e == cudaSuccess ? launch_edt_pass(d_vox, d_scratch, scratch_words, d, 2, s, cfg.rows) : e;
+  return launch_sweeps(d_vox, d_scratch, scratch_words, d, s, cfg, nullptr);
 }
 
 // The occupancy-bit pass Z over a batch (one persistent launch); skip_other:
@@ -1608,43 +1671,52 @@ cudaError_t launch_z_bits_batch(const BatchMap* d_table, const BatchItems& it, c
 
 cudaError_t launch_voxelize_edt_batch(const BatchMap* d_table, const BatchItems& it, const float* d_xyz,
                                       const uint64_t* d_offsets, uint64_t n_total, cudaStream_t s, int rows) {
+  cudaError_t e;
+  if (it.search) {  // no slice waits: only the error word is cleared
+    e = cudaMemsetAsync(it.d_sync + it.sync_words, 0, 2 * sizeof(unsigned), s);
+    return e == cudaSuccess ? launch_search_voxelize_batch(d_table, it, d_xyz, d_offsets, n_total, s) : e;
+  }
   occ_clear_batch_kernel<<<dim3(64, it.n_maps), 256, 0, s>>>(d_table);
-  cudaError_t e = cudaGetLastError();
-  if (e != cudaSuccess) return e;
+  if ((e = cudaGetLastError()) != cudaSuccess) return e;
   if (n_total > 0) {
     const unsigned blocks = (unsigned)std::min<uint64_t>((n_total + 255) / 256, (uint64_t)device_sms() * 16);
     occ_insert_batch_kernel<<<blocks, 256, 0, s>>>(d_table, it.n_maps, d_xyz, d_offsets, n_total);
     if ((e = cudaGetLastError()) != cudaSuccess) return e;
   }
   if ((e = launch_z_bits_batch(d_table, it, s, 0)) != cudaSuccess) return e;
-  return (rows == 0 ? sweep_rows() : rows) == 32 ? launch_yx_batch<32>(d_table, it, s)
-                                                 : launch_yx_batch<16>(d_table, it, s);
+  return (rows == 0 ? sweep_rows() : rows) == 32 ? launch_yx_batch<32>(d_table, it, s, 0)
+                                                 : launch_yx_batch<16>(d_table, it, s, 0);
 }
 
 // Batched EDT of filled maps.  Pass Z as for one map: each map's occupancy
 // bits and other-sites flag from its voxels, then the bits pass for the maps
 // whose voxels are all UNINIT or their own sites and the general pass for the
-// others (each launch skips the other maps).
+// others (each launch skips the other maps).  Where the row search takes every
+// map it replaces the bits pass and the sweeps of the first kind.
 cudaError_t launch_edt_batch(const BatchMap* d_table, const BatchItems& it, cudaStream_t s, int rows) {
   batch_flags_clear_kernel<<<(it.n_maps + 255) / 256, 256, 0, s>>>(d_table, it.n_maps);
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return e;
-  int per_sm = 0;
-  if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, occ_from_map_batch_kernel, 256, 0)) != cudaSuccess)
-    return e;
-  const long long occ_blocks = std::max<long long>(
-      1, std::min<long long>((it.total[3] + 7) / 8, (long long)device_sms() * std::max(per_sm, 1)));
-  occ_from_map_batch_kernel<<<(unsigned)occ_blocks, 256, 0, s>>>(d_table, it.d_prefix[3], it.n_maps, it.total[3]);
-  if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  if ((e = launch_z_bits_batch(d_table, it, s, 1)) != cudaSuccess) return e;
+  if (it.search) {
+    if ((e = launch_search_filled_batch(d_table, it, s)) != cudaSuccess) return e;
+  } else {
+    int per_sm = 0;
+    if ((e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, occ_from_map_batch_kernel, 256, 0)) != cudaSuccess)
+      return e;
+    const long long occ_blocks = std::max<long long>(
+        1, std::min<long long>((it.total[3] + 7) / 8, (long long)device_sms() * std::max(per_sm, 1)));
+    occ_from_map_batch_kernel<<<(unsigned)occ_blocks, 256, 0, s>>>(d_table, it.d_prefix[3], it.n_maps, it.total[3]);
+    if ((e = cudaGetLastError()) != cudaSuccess) return e;
+    if ((e = launch_z_bits_batch(d_table, it, s, 1)) != cudaSuccess) return e;
+  }
   const int smem = kZWarps * kZWarpWords * 4;
   long long blocks = 0;
   if ((e = kernel_setup<edt_pass_z_batch>(kZWarps * 32, smem, &blocks)) != cudaSuccess) return e;
   blocks = std::max<long long>(1, std::min<long long>(blocks, (it.total[0] + kZWarps - 1) / kZWarps));
   edt_pass_z_batch<<<(unsigned)blocks, kZWarps * 32, smem, s>>>(d_table, it.d_prefix[0], it.n_maps, it.total[0]);
   if ((e = cudaGetLastError()) != cudaSuccess) return e;
-  return (rows == 0 ? sweep_rows() : rows) == 32 ? launch_yx_batch<32>(d_table, it, s)
-                                                 : launch_yx_batch<16>(d_table, it, s);
+  return (rows == 0 ? sweep_rows() : rows) == 32 ? launch_yx_batch<32>(d_table, it, s, it.search)
+                                                 : launch_yx_batch<16>(d_table, it, s, it.search);
 }
 
 }  // namespace gvx

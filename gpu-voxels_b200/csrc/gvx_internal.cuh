@@ -92,6 +92,10 @@ struct gvx_blist {
 
 namespace gvx {
 
+// Words of the EDT workspace's counter area (Z slice counters, queue head,
+// error word, pass Z's other-sites flag, padded to 32).
+__host__ __device__ __forceinline__ uint64_t edt_sync_words(int Z) { return ((uint64_t)Z + 3 + 31) / 32 * 32; }
+
 // One map of a batch, as the batched kernels see it.
 struct BatchMap {
   uint32_t* vox;
@@ -104,19 +108,21 @@ struct BatchMap {
 
 // Work-item layout of the batched EDT: for pass p, map k owns warp items
 // [prefix[p][k], prefix[p][k+1]); prefix[3] numbers the occupancy-bit tasks
-// of pass Z on filled maps (32 columns x 32 rows each).  The fused Y -> X launch keeps one stack of
+// of pass Z on filled maps (32 columns x 32 rows each), prefix[4] and
+// prefix[5] the row search's blocks of passes Y and X.  The fused Y -> X launch keeps one stack of
 // stack_len rows (64 words each) per resident warp in d_stacks and its slice
 // counters, queue head and error word in d_sync (sync_words + 2 words).
 struct BatchItems {
-  long long* d_prefix[4];
-  long long total[4];
+  long long* d_prefix[6];
+  long long total[6];
   uint32_t n_maps;
   uint32_t* d_stacks;
   long long stack_warps;
   uint32_t stack_len;
   unsigned* d_sync;
   unsigned sync_words;
-  uint32_t z_max;  // the tallest map's Z
+  uint32_t x_max, y_max, z_max;  // the largest dims of any map
+  bool search;  // the row search takes every map
 };
 
 // Error reporting shared by the ABI units.
@@ -154,6 +160,23 @@ cudaError_t launch_edt(uint32_t* d_vox, uint32_t* d_scratch, uint64_t scratch_wo
 // pass when a voxel holds another site), 1 = Y, 2 = X, 3 = fused Y -> X
 cudaError_t launch_edt_pass(uint32_t* d_vox, uint32_t* d_scratch, uint64_t scratch_words, gvx_dims d, int pass,
                             cudaStream_t s, int rows = 0);
+// The row search (edt_search.cu): the EDT of maps whose sites are all their own
+// voxels, for dims it takes.  area: search_words(d) words, the first
+// search_bits_words(d) of them occupancy bits (zeroed by the caller before
+// launch_search_voxelize).  launch_search_filled sets *d_other (zeroed by the
+// caller) and leaves the map as it is when a voxel holds another site.
+bool search_takes(gvx_dims d);
+uint64_t search_words(gvx_dims d);
+uint64_t search_bits_words(gvx_dims d);
+cudaError_t launch_search_voxelize(uint32_t* d_vox, uint32_t* area, gvx_dims d, float side, const float* d_xyz, uint64_t n,
+                                   uint32_t* d_outside, cudaStream_t s);
+cudaError_t launch_search_filled(uint32_t* d_vox, uint32_t* area, gvx_dims d, uint32_t* d_other, cudaStream_t s);
+// Blocks of pass 1 (Y) or 2 (X) for a map.
+long long search_items(gvx_dims d, int pass);
+// The same over every map of a batch whose maps it all takes (BatchItems::search).
+cudaError_t launch_search_voxelize_batch(const BatchMap* d_table, const BatchItems& it, const float* d_xyz,
+                                         const uint64_t* d_offsets, uint64_t n_total, cudaStream_t s);
+cudaError_t launch_search_filled_batch(const BatchMap* d_table, const BatchItems& it, cudaStream_t s);
 // Synchronous read of the error word the last fused launch left (0 = ok).
 cudaError_t edt_read_error(const uint32_t* d_scratch, gvx_dims d, uint32_t* flag);
 // BitVoxelMap bit maintenance: clear `bits` (8 words) in every voxel; move

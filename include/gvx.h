@@ -101,14 +101,16 @@ GVX_API gvx_status gvx_dvm_voxelize_edt(gvx_dvm *m, const float *d_xyz, uint64_t
  * every voxel is UNINIT or its own site: occupancy bits read from the map,
  * then the sweep over the bits; otherwise the general sweep), 1 = the y sweep,
  * 2 = the x sweep (one launch each), 3 = the y and x sweeps
- * as the single fused launch gvx_dvm_edt uses, which takes pass 0's output
+ * as one fused launch (gvx_dvm_edt's where it sweeps), which takes pass 0's output
  * and its record of the route it took (0 then 3 == gvx_dvm_edt;
  * 0, 1, 2 gives the same result).  Pass 0 alone equals the reference's
  * phase 1 (kernelPBAphase1FloodZ, GV/voxelmap/kernels/VoxelMapOperationsPBA.hpp:63-124). */
 GVX_API gvx_status gvx_dvm_edt_pass(gvx_dvm *m, int pass, gvx_stream stream);
 /* EDT launch configuration chosen by the autotuner: rows per staging chunk of
  * the sweeps (16 or 32; 0 = library default), whether the y and x sweeps run
- * as one fused launch (1) or two (0), and the time measured for it. */
+ * as one fused launch (1) or two (0), and the time measured for it.  The sweeps
+ * run for maps longer than 512 in x or y and for maps holding sites outside
+ * their own voxels; the other maps' EDT (a search per row) has no setting. */
 typedef struct {
   uint32_t rows;
   uint32_t fused;
@@ -252,8 +254,8 @@ GVX_API gvx_status gvx_batch_clear(gvx_batch *b, gvx_stream stream);
 /* Points of all maps concatenated; map k owns points [d_offsets[k], d_offsets[k+1]). */
 GVX_API gvx_status gvx_batch_insert_points(gvx_batch *b, const float *d_xyz, const uint64_t *d_offsets, uint64_t n_total,
                                            gvx_stream stream);
-/* EDT of every map, bit-identical to gvx_dvm_edt per map: one launch for the
- * z sweeps of all maps, one fused launch for their y and x sweeps. */
+/* EDT of every map, bit-identical to gvx_dvm_edt per map: one launch per step
+ * over all maps. */
 GVX_API gvx_status gvx_batch_edt(gvx_batch *b, gvx_stream stream);
 /* gvx_batch_clear + gvx_batch_insert_points + gvx_batch_edt in one call, as
  * gvx_dvm_voxelize_edt per map (this is what a captured graph records). */

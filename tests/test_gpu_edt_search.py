@@ -1,0 +1,96 @@
+"""The row search (csrc/edt_search.cu) against the oracle's EDT, bit for bit, at the sizes where its tiles end:
+segments of 16 rows times 8 warps (16, 128, 256, 384, 512), 4-candidate rounds, 32-z chunks, rows whose length is a
+multiple of 4 (16-byte stores) and not, columns longer than 512 (the sweeps take the map), and scenes from a few
+sites (long jumps between winners) to nearly full."""
+import numpy as np
+import pytest
+import torch
+
+import gvx
+import oracle
+from gpu_helpers import first_mismatch, oracle_edt, to_u32
+from gvx.batch import Batch
+
+SIDE = 0.01
+
+
+def _points(dims, n, seed):
+    rng = np.random.default_rng(seed)
+    v = np.stack([rng.integers(0, d, n) for d in dims], 1)
+    return ((v + rng.uniform(0.1, 0.9, v.shape)) * SIDE).astype(np.float32)
+
+
+def _floor(dims, seed):
+    """A rough floor and a far wall: every column has sites, winners jump between the two."""
+    rng = np.random.default_rng(seed)
+    x, y = np.meshgrid(np.arange(dims[0]), np.arange(dims[1]), indexing="ij")
+    z = np.clip(dims[2] // 8 + rng.integers(-1, 2, x.shape), 0, dims[2] - 1)
+    p = np.stack([x, y, z], -1).reshape(-1, 3)
+    wall = np.stack([np.full(dims[1], dims[0] - 1), np.arange(dims[1]), np.full(dims[1], dims[2] // 2)], 1)
+    return ((np.concatenate([p, wall]) + 0.5) * SIDE).astype(np.float32)
+
+
+DIMS = [(1, 1, 1), (15, 17, 31), (16, 16, 32), (33, 31, 33), (127, 129, 40), (128, 128, 64), (130, 20, 65),
+        (255, 257, 9), (384, 12, 34), (13, 385, 32), (511, 10, 33), (12, 512, 31), (512, 512, 5), (513, 9, 40),
+        (9, 513, 20), (20, 24, 600), (21, 9, 1023), (64, 48, 1)]
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims", DIMS)
+@pytest.mark.parametrize("scene", ["none", "one", "few", "some", "dense", "floor"])
+def test_search_equals_oracle(dims, scene):
+    n = dims[0] * dims[1] * dims[2]
+    count = {"none": 0, "one": 1, "few": 7, "some": max(1, n // 100), "dense": max(1, n // 2), "floor": 0}[scene]
+    pts = _floor(dims, n) if scene == "floor" else _points(dims, min(count, 400_000), n + count)
+    _, want = oracle_edt(dims, SIDE, pts)
+    m = gvx.DistanceVoxelMap(dims, SIDE)
+    p = torch.as_tensor(pts)
+    m.voxelize_edt(p)
+    got = to_u32(m.data())
+    assert np.array_equal(got, want), first_mismatch(got, want, dims)
+    m.clearMap()
+    m.insertPointCloud(p)
+    m.parallelBanding3D()
+    got = to_u32(m.data())
+    assert np.array_equal(got, want), first_mismatch(got, want, dims)
+    assert m.edt_check() == 0
+
+
+@pytest.mark.gpu
+def test_search_leaves_other_sites_to_the_sweeps():
+    """A map transformed before holds other sites than its voxels' own: the second EDT equals the oracle's second."""
+    dims = (70, 65, 50)
+    pts = _points(dims, 300, 5)
+    _, want = oracle_edt(dims, SIDE, pts)
+    m = gvx.DistanceVoxelMap(dims, SIDE)
+    m.insertPointCloud(torch.as_tensor(pts))
+    for _ in range(2):
+        m.parallelBanding3D()
+        got = to_u32(m.data())
+        assert np.array_equal(got, want), first_mismatch(got, want, dims)
+        oracle.pba(want, dims)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("long_map", [False, True])
+def test_batch_search_equals_oracle(long_map):
+    """Uneven maps in one batch, one of them transformed before its turn; with a column above 512 rows in the batch
+    the sweeps take every map."""
+    dims = [(40, 33, 70), (129, 16, 31), (16, 200, 33), (1, 1, 1), (65, 64, 96)] + ([(520, 8, 9)] if long_map else [])
+    clouds = [_points(d, max(1, d[0] * d[1] * d[2] // 200), i) for i, d in enumerate(dims)]
+    maps = [gvx.DistanceVoxelMap(d, SIDE) for d in dims]
+    b = Batch(maps)
+    xyz = torch.as_tensor(np.concatenate(clouds)).cuda()
+    offsets = torch.tensor(np.concatenate([[0], np.cumsum([len(c) for c in clouds])]), dtype=torch.int64).cuda()
+    wants = [oracle_edt(d, SIDE, c)[1] for d, c in zip(dims, clouds)]
+    b.voxelize_edt(xyz, offsets)
+    for m, d, w in zip(maps, dims, wants):
+        assert np.array_equal(to_u32(m.data()), w), first_mismatch(to_u32(m.data()), w, d)
+    b.clear()
+    b.insert(xyz, offsets)
+    maps[0].parallelBanding3D()  # this one comes transformed
+    oracle.pba(wants[0], dims[0])
+    b.edt()
+    for m, d, w in zip(maps, dims, wants):
+        assert np.array_equal(to_u32(m.data()), w), first_mismatch(to_u32(m.data()), w, d)
+    assert b.edt_check() == 0
