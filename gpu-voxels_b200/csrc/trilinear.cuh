@@ -81,8 +81,13 @@ __device__ __forceinline__ void axis_setup(float p, float side, int n, int& i0, 
 // kinematics): cell and fraction come from p / side - 0.5 in double, so only
 // the fraction (in [0, 1]) is rounded to float -- an FP32 position alone would
 // carry up to half an ulp of p (1.2e-5 voxel at 2.56 m with 1 cm voxels).
-__device__ __forceinline__ void axis_setup(double p, float side, int n, int& i0, int& i1, float& f, bool& free_axis) {
-  const double u = p / (double)side - 0.5;
+// inv = 1 / side: the quotient is p * inv with one residual correction
+// (P. Markstein, IBM J. Res. Develop. 34(1), 1990) in place of three FP64
+// divides per point.
+__device__ __forceinline__ void axis_setup(double p, float side, double inv, int n, int& i0, int& i1, float& f,
+                                           bool& free_axis) {
+  const double q0 = p * inv;
+  const double u = (fabs(q0) < 1e300 ? fma(fma(-q0, (double)side, p), inv, q0) : q0) - 0.5;  // an infinity stays one
   const double hi = (double)(n - 1);
   free_axis = (u >= 0.0) && (u <= hi);
   const double uc = fmin(fmax(u, 0.0), hi);  // NaN -> 0
@@ -96,15 +101,20 @@ struct Tri {
   float gx, gy, gz;  // d(distance)/d(position), dimensionless
 };
 
-// Trilinear distance and gradient at a position given in float or double.
+__device__ __forceinline__ void axis_setup(float p, float side, float, int n, int& i0, int& i1, float& f, bool& free_axis) {
+  axis_setup(p, side, n, i0, i1, f, free_axis);
+}
+
+// Trilinear distance and gradient at a position given in float or double (inv
+// = 1 / side, used for a double).
 template <class Real>
-__device__ __forceinline__ Tri trilinear(const MapView& m, Real px, Real py, Real pz) {
+__device__ __forceinline__ Tri trilinear(const MapView& m, Real px, Real py, Real pz, Real inv = Real(0)) {
   int i0, i1, j0, j1, k0, k1;
   float fx, fy, fz;
   bool ax, ay, az;
-  axis_setup(px, m.side, m.X, i0, i1, fx, ax);
-  axis_setup(py, m.side, m.Y, j0, j1, fy, ay);
-  axis_setup(pz, m.side, m.Z, k0, k1, fz, az);
+  axis_setup(px, m.side, inv, m.X, i0, i1, fx, ax);
+  axis_setup(py, m.side, inv, m.Y, j0, j1, fy, ay);
+  axis_setup(pz, m.side, inv, m.Z, k0, k1, fz, az);
   float d000, d100, d010, d110, d001, d101, d011, d111;
   corner_pair(m, i0, i1, j0, k0, d000, d100);
   corner_pair(m, i0, i1, j1, k0, d010, d110);
