@@ -556,6 +556,7 @@ gvx_status gvx_blist_data(const gvx_blist* l, uint32_t** d_ids, uint8_t** d_voxe
 gvx_status gvx_blist_clear(gvx_blist* l) {
   if (l == nullptr) return fail(GVX_ERR_INVALID_ARG, "list is null");
   l->n = 0;
+  l->in_map = true;
   return GVX_OK;
 }
 
@@ -669,6 +670,54 @@ cudaError_t blist_spare(gvx_blist* l, uint64_t cap) {
 
 inline size_t align256(size_t b) { return (b + 255) & ~(size_t)255; }
 
+// The merged list becomes the list; the old storage is the next call's spare.
+void blist_adopt_spare(gvx_blist* l, uint64_t n) {
+  std::swap(l->d_ids, l->d_ids2);
+  std::swap(l->d_vox, l->d_vox2);
+  std::swap(l->cap, l->cap2);
+  l->n = n;
+}
+
+// Whether a list is built by the bitmap of its reference map (list_bits.cu)
+// rather than by a sort: its cost and its memory grow with the map (4 bytes
+// per 32 voxels, twice that when the list already has entries), the sort's
+// with the points.  Up to 2^20 words (320^3 voxels, 4 MB, a few microseconds
+// per pass over them) it is the faster at any length (200k points at 256^3:
+// 119 us with the collision and the read-back, by sort 214); beyond, it may
+// take 64 bytes per entry, less than three times the sort's work area.
+bool list_by_bits(const gvx_blist* l, uint64_t total) {
+  return l->in_map && (num_voxels(l->ref) + 31) / 32 <= (1ull << 20) + 16 * total;
+}
+
+// Entries whose storage is taken at the upper bound (every old entry and
+// point its own voxel) so that the merged length need not be waited for
+// before the list is written: 36 bytes each.
+constexpr uint64_t kUpperBoundEntries = 1ull << 20;
+
+gvx_status blist_insert_by_bits(gvx_blist* l, const float* d_xyz, uint64_t n, uint32_t meaning, cudaStream_t s) {
+  const uint64_t total = l->n + n;
+  cudaError_t e = grow(&l->d_work, &l->work_bytes, list_bits_work_words(l->ref, l->n, n) * sizeof(uint32_t));
+  if (e != cudaSuccess) return cuda_status(e, "list insert buffers");
+  uint32_t* work = static_cast<uint32_t*>(l->d_work);
+  const uint32_t* d_total = nullptr;
+  uint32_t n_out = 0;
+  e = launch_list_mark(work, l->ref, l->side, d_xyz, n, l->d_ids, l->n, &d_total, s);
+  const uint64_t bound = std::min<uint64_t>(total, num_voxels(l->ref));
+  if (e == cudaSuccess && bound <= kUpperBoundEntries) {
+    e = blist_spare(l, bound);
+  } else if (e == cudaSuccess) {
+    e = cudaMemcpyAsync(&n_out, d_total, sizeof(n_out), cudaMemcpyDeviceToHost, s);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // the merged list's length sizes its storage
+    if (e == cudaSuccess) e = blist_spare(l, n_out);
+  }
+  if (e == cudaSuccess) e = launch_list_emit(work, l->ref, n, l->d_ids, l->d_vox, l->n, meaning, l->d_ids2, l->d_vox2, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&n_out, d_total, sizeof(n_out), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // blocking, as the reference's insert
+  if (e != cudaSuccess) return cuda_status(e, "list insert");
+  blist_adopt_spare(l, n_out);
+  return GVX_OK;
+}
+
 }  // namespace
 }  // namespace gvx
 
@@ -681,6 +730,7 @@ gvx_status gvx_blist_insert_points(gvx_blist* l, const float* d_xyz, uint64_t n,
   cudaStream_t s = as_stream(stream);
   const uint64_t total = l->n + n;
   if (total >= 0xFFFFFFFFull) return fail(GVX_ERR_OUT_OF_DOMAIN, "list too long");
+  if (list_by_bits(l, total)) return blist_insert_by_bits(l, d_xyz, n, meaning, s);
   // work area: keys, vals, sorted keys, sorted vals, run heads, run positions
   // (total words each), then CUB's temporary storage
   size_t sort_bytes = 0, scan_bytes = 0;
@@ -718,11 +768,7 @@ gvx_status gvx_blist_insert_points(gvx_blist* l, const float* d_xyz, uint64_t n,
   e = cudaGetLastError();
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // blocking, as the reference's insert
   if (e != cudaSuccess) return cuda_status(e, "list merge");
-  // the merged list becomes the list; the old storage is the next call's spare
-  std::swap(l->d_ids, l->d_ids2);
-  std::swap(l->d_vox, l->d_vox2);
-  std::swap(l->cap, l->cap2);
-  l->n = n_out;
+  blist_adopt_spare(l, n_out);
   return GVX_OK;
 }
 
@@ -732,6 +778,7 @@ gvx_status gvx_blist_set(gvx_blist* l, const uint32_t* d_ids, const uint8_t* d_v
   if (meaning > 255) return fail(GVX_ERR_INVALID_ARG, "meaning must be in [0, 255]");
   cudaStream_t s = as_stream(stream);
   l->n = 0;
+  l->in_map = n == 0;
   cudaError_t e = blist_reserve(l, n, s);
   if (e != cudaSuccess) return cuda_status(e, "list storage");
   if (n == 0) return GVX_OK;
@@ -822,6 +869,7 @@ gvx_status gvx_extract_given_distances(const gvx_dvm* m, int min_dist, int max_d
   if (e == cudaSuccess) e = cudaMemcpyAsync(&total, tiles + nt, sizeof(uint32_t), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);
   result->n = 0;
+  result->in_map = true;
   if (e == cudaSuccess) e = blist_reserve(result, total, s);
   if (e == cudaSuccess && total > 0) e = launch_band_write(m->d_vox, m->dims, min_dist, max_dist, tiles, result->d_ids,
                                                            result->d_vox, s);
