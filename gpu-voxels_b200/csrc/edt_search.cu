@@ -23,21 +23,22 @@
 // (x) plane for pass Y and of one (y) plane for pass X, all keys in shared
 // memory (key[row][lane], no bank conflicts).  Its 8 warps first find the
 // winners at 8 rows (segment_starts), then each warp refines its eighth of the
-// column to every 16th, every 8th and every row, with one add-and-min per
-// candidate and row.  The lanes of a warp share the candidate range (the union of theirs):
+// column to every 8th row and then to every row, with one add-and-min per
+// candidate and row (a step by 16 rows between the two was 8 % slower: more
+// loops, each with its own range to find).  The lanes of a warp share the candidate range (the union of theirs):
 // neighbours in z see nearly the same obstacles, so the union is 1.06 .. 1.27
 // times a lane's own range at the coarse steps and about 1.7 times at the last
 // (512^3 depth scene); with lanes along x, as the sweeps have them, it was up to
 // 7.9 times.
 //
-// What bounds it: instruction issue, then the 2-cycle integer pipe (a candidate
-// costs one add-and-min, no divide, no per-lane control flow); DRAM is a third
-// busy.  Measured on a B200, this pass against the sweeps of edt.cu
-// (voxelize_edt, warm): 512^3 depth scene 839 us against 1710 (pass Y 361, pass
-// X 447); 128^3 with 50k box points 45 against 183 (the sweeps walk 128 rows
-// one after another per pass, here 8 warps share a column); 203 x 331 x 157 in
-// three calls 168 against 491; 24 uneven maps of 64 to 384 per axis in one
-// batch 1780 against 2606.
+// What bounds it: instruction issue and the 2-cycle integer pipe (65 % and 70 %
+// busy; a candidate costs one add-and-min, no divide, no per-lane control
+// flow); DRAM is a third busy.  Measured on a B200 against the sweeps of edt.cu
+// (whole calls, warm): 512^3 depth scene 810 us against 1710 (pass Y 358, pass X
+// 440); 128^3 with 50k box points 37 against 183 (the sweeps walk 128 rows one
+// after another per pass, here 8 warps share a column); 203 x 331 x 157 in three
+// calls 145 against 491; 24 uneven maps of 64 to 384 per axis in one batch 1551
+// against 2606.
 //
 // The searching loops are kept rolled: unrolled over a warp's rows the code
 // outgrew the instruction caches (at 352^3 the largest stall was 'no
@@ -54,6 +55,7 @@
 
 #include <algorithm>
 #include <mutex>
+#include <type_traits>
 
 #include "gvx_internal.cuh"
 
@@ -125,6 +127,15 @@ __device__ __forceinline__ Search search_setup(uint32_t* smem, int L, uint32_t**
 // candidate's row).
 __device__ __forceinline__ uint32_t shift_key(uint32_t k, int d2, int i) { return k + (uint32_t)((d2 + i) * i) * 1024u; }
 
+// The least of `best` and four candidates at their weights.
+__device__ __forceinline__ uint32_t least_of(const uint32_t (&c)[4], uint32_t d0, uint32_t d1, uint32_t d2, uint32_t d3,
+                                             uint32_t best) {
+  best = __viaddmin_u32(c[0], d0, best);
+  best = __viaddmin_u32(c[1], d1, best);
+  best = __viaddmin_u32(c[2], d2, best);
+  return __viaddmin_u32(c[3], d3, best);
+}
+
 // Candidates against the rows r0 + kStep * {1 .. kN}, r0 a multiple of 8:
 // best[i] = the least key.  lo2, hi2: twice the first and the last candidate
 // (warp-uniform); some: all ones, 0 in a column without a site.  Four
@@ -139,9 +150,7 @@ template <int kStep, int kN>
 __device__ __forceinline__ void refine(const Search& s, int r0, int lo2, int hi2, uint32_t some, uint32_t (&best)[kN]) {
 #pragma unroll
   for (int i = 0; i < kN; ++i) best[i] = 0xffffffffu;
-  auto round = [&](int j2) {
-    const uint32_t* k = s.key + j2 * 16;
-    const uint32_t* w = s.w + (r0 - (j2 >> 1));
+  auto round = [&](const uint32_t* k, const uint32_t* w) {
     const uint32_t c[4] = {k[0], k[32], k[64], k[96]};
     if constexpr (kStep == 1) {  // the (row, candidate) differences of a round are consecutive
       uint32_t d[12];
@@ -151,38 +160,43 @@ __device__ __forceinline__ void refine(const Search& s, int r0, int lo2, int hi2
         d[4 * g] = v.x, d[4 * g + 1] = v.y, d[4 * g + 2] = v.z, d[4 * g + 3] = v.w;
       }
 #pragma unroll
-      for (int i = 0; i < kN; ++i) {
-#pragma unroll
-        for (int t = 0; t < 4; ++t) best[i] = __viaddmin_u32(c[t], d[i + 4 - t], best[i]);
-      }
+      for (int i = 0; i < kN; ++i) best[i] = least_of(c, d[i + 4], d[i + 3], d[i + 2], d[i + 1], best[i]);
     } else {
 #pragma unroll
       for (int i = 0; i < kN; ++i) {
         const uint4 v = *reinterpret_cast<const uint4*>(w + kStep * (i + 1) - 3);
-        best[i] = __viaddmin_u32(c[0], v.w, best[i]);
-        best[i] = __viaddmin_u32(c[1], v.z, best[i]);
-        best[i] = __viaddmin_u32(c[2], v.y, best[i]);
-        best[i] = __viaddmin_u32(c[3], v.x, best[i]);
+        best[i] = least_of(c, v.w, v.z, v.y, v.x, best[i]);
       }
     }
   };
   lo2 &= ~7;
-  const bool jump = hi2 - lo2 >= 80;
-  if (jump) round(hi2 & ~7);
+  if (hi2 - lo2 < 80) {
+    const uint32_t* k = s.key + lo2 * 16;
+    const uint32_t* w = s.w + (r0 - (lo2 >> 1));
+    const uint32_t* const k_end = s.key + hi2 * 16;
 #pragma unroll 1
-  for (; lo2 <= hi2; lo2 += 8) {
-    if (jump && (lo2 & 31) == 0) {
+    for (; k <= k_end; k += 128, w -= 4) round(k, w);
+    return;
+  }
+  int j2 = hi2 & ~7;  // the far end first
+  bool far_end = true;
+#pragma unroll 1
+  while (true) {
+    round(s.key + j2 * 16, s.w + (r0 - (j2 >> 1)));
+    j2 = far_end ? lo2 : j2 + 8;
+    far_end = false;
+    if (j2 > hi2) break;
+    if ((j2 & 31) == 0) {
       uint32_t limit = best[0];
 #pragma unroll
       for (int i = 1; i < kN; ++i) limit = max(limit, best[i]);
       limit &= some;
 #pragma unroll 1
-      for (; lo2 + 32 <= hi2; lo2 += 32) {
-        const int first = lo2 >> 1, gap = max(max(r0 + kStep - first - 15, first - r0 - kN * kStep), 0);
-        if (__any_sync(kFullMask, ((uint32_t)s.least[lo2] << 15) + s.w[gap] <= limit)) break;
+      for (; j2 + 32 <= hi2; j2 += 32) {
+        const int first = j2 >> 1, gap = max(max(r0 + kStep - first - 15, first - r0 - kN * kStep), 0);
+        if (__any_sync(kFullMask, ((uint32_t)s.least[j2] << 15) + s.w[gap] <= limit)) break;
       }
     }
-    round(lo2);
   }
 }
 
@@ -292,52 +306,59 @@ __device__ __forceinline__ void search_rows(const Search& s, Out& out) {
     lo2 = (int)__reduce_min_sync(kFullMask, (klo & kRowBits) | or_lo);
     hi2 = (int)__reduce_max_sync(kFullMask, khi & and_hi);
   };
-  uint32_t n[3] = {end, end, end}, n3 = end;  // winners at the ends of the 16-row groups
-  if (S > 16) {
-    range(cur, end);
-    if (lo2 >= hi2) {
+  uint32_t n[8];  // winners at the ends of the 8-row groups
+  auto group_ends = [&](auto rows) {
+    constexpr int kN = decltype(rows)::value;
+    uint32_t b[kN];
+    refine<8, kN>(s, seg0, lo2, hi2, some, b);
 #pragma unroll
-      for (int i = 0; i < 3; ++i) n[i] = shift_key(cur, 2 * seg0 - lo2, 16 * (i + 1));
-    } else {
-      refine<16, 3>(s, seg0, lo2, hi2, some, n);
-    }
-    if (S <= 32) n[1] = end;
-    if (S <= 48) n[2] = end;
+    for (int i = 0; i < 8; ++i) n[i] = i < kN ? b[i < kN ? i : 0] : end;
+  };
+  range(cur, end);
+  if (lo2 >= hi2) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) n[i] = 8 * i + 8 < S ? shift_key(cur, 2 * seg0 - lo2, 8 * (i + 1)) : end;
+  } else if (S == 16) {
+    group_ends(std::integral_constant<int, 1>{});
+  } else if (S == 32) {
+    group_ends(std::integral_constant<int, 3>{});
+  } else if (S == 48) {
+    group_ends(std::integral_constant<int, 5>{});
+  } else {
+    group_ends(std::integral_constant<int, 7>{});
   }
 #pragma unroll 1
-  for (int r0 = seg0; r0 < seg1; r0 += 16) {
-    const uint32_t nxt = r0 + 16 < s.L ? n[0] : last;
-    range(cur, nxt);
-    if (lo2 >= hi2) {  // one site (or none) for all 16 rows
-      out.same16(r0, cur, 2 * r0 - lo2);
-    } else {
-      uint32_t mid[1];
-      refine<8, 1>(s, r0, lo2, hi2, some, mid);
-      uint32_t up = r0 + 8 < s.L ? mid[0] : last;
-#pragma unroll 1
-      for (int r = r0; r < min(r0 + 16, s.L); r += 8) {
-        uint32_t b[7];
-        range(cur, up);
-        const bool same = lo2 >= hi2;
-        if (same) {
+  for (int r = seg0; r < seg1; r += 8) {
+    uint32_t b[7];
+    range(cur, r + 8 < s.L ? n[0] : last);
+    const bool same = lo2 >= hi2;
+    if (same) {
 #pragma unroll
-          for (int i = 0; i < 7; ++i) b[i] = shift_key(cur, 2 * r - lo2, i + 1);
-        } else {
-          refine<1, 7>(s, r, lo2, hi2, some, b);
-        }
-        const uint32_t o[8] = {cur, b[0], b[1], b[2], b[3], b[4], b[5], b[6]};
-        out.rows(r, o, same);
-        cur = mid[0];
-        up = nxt;
-      }
+      for (int i = 0; i < 7; ++i) b[i] = shift_key(cur, 2 * r - lo2, i + 1);
+    } else {
+      refine<1, 7>(s, r, lo2, hi2, some, b);
     }
-    cur = nxt;
-    n[0] = n[1];
-    n[1] = n[2];
-    n[2] = n3;
+    const uint32_t o[8] = {cur, b[0], b[1], b[2], b[3], b[4], b[5], b[6]};
+    out.rows(r, o, same);
+    cur = n[0];
+#pragma unroll
+    for (int i = 0; i < 7; ++i) n[i] = n[i + 1];
   }
   out.finish();
 }
+
+// ---------------------------------------------------------------------------
+// Launches of a step chain (programmatic dependent launch): a kernel's blocks
+// may take their places while the one before drains.  wait_for_previous comes
+// before the first access to what that kernel wrote -- it returns once the
+// previous kernel has ended and its writes are visible -- and start_next once a
+// block needs nothing more from the launch order.  Two kernels before the
+// current one are complete as well: the previous one waited for them.  With
+// the rolled loops above this took 128^3 with queries from 45 to 37 us and
+// 203 x 331 x 157 from 168 to 145.
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void start_next() { asm volatile("griddepcontrol.launch_dependents;"); }
 
 struct OutY {
   uint32_t* out;  // row 0 of this lane's column in `field`
@@ -349,14 +370,6 @@ struct OutY {
     for (int i = 0; i < 8; ++i, o += (uint32_t)X * 32u)
       if (r + i < Y) *o = k[i];
   }
-  __device__ __forceinline__ void same16(int r0, uint32_t k, int d2) {
-    uint32_t* o = out + (uint32_t)(r0 * X) * 32u;
-#pragma unroll 4
-    for (int r = r0; r < min(r0 + 16, Y); ++r, d2 += 2, o += (uint32_t)X * 32u) {
-      *o = k;
-      k = shift_key(k, d2, 1);
-    }
-  }
   __device__ __forceinline__ void finish() {}
 };
 
@@ -366,6 +379,8 @@ __device__ __forceinline__ void item_y(uint32_t* smem, const uint32_t* __restric
   const int lane = threadIdx.x & 31;
   uint32_t* extra;
   const Search s = search_setup(smem, Y, &extra);
+  start_next();
+  wait_for_previous();
   uint2* col = reinterpret_cast<uint2*>(extra);  // (bits, near) of every y
   const uint64_t base = ((uint64_t)c * X + x) * Y;
   for (int y = threadIdx.x; y < Y; y += kWarps * 32) col[y] = make_uint2(__ldg(bits + base + y), __ldg(near + base + y));
@@ -377,15 +392,15 @@ __device__ __forceinline__ void item_y(uint32_t* smem, const uint32_t* __restric
   // (only possible when Z is above 512).  A thread makes the keys of 4
   // consecutive z: where the chunk holds no site of the column, a square's
   // step to the next z is one addition.
-  const int l = 4 * (threadIdx.x & 7);
-  const bool plain = Z <= 512 && c * 32 + 32 <= Z;
+  const int l = 4 * (threadIdx.x & 7), z0 = c * 32 + l;
   uint4* keys = reinterpret_cast<uint4*>(smem) + threadIdx.x;
 #pragma unroll 1
-  for (int y = threadIdx.x >> 3; y < Y; y += kWarps * 4, keys += kWarps * 32) {
+  for (int y0 = (threadIdx.x >> 5) * 4; y0 < Y; y0 += kWarps * 4, keys += kWarps * 32) {  // four y per warp
+    const int y = min(y0 + (lane >> 3), Y - 1);
     const uint2 q = col[y];
     int below = (int)(short)(q.y & 0xffffu), above = (int)q.y >> 16;
     uint32_t k[4];
-    if (plain && q.x == 0u) {
+    if (Z <= 512 && !__any_sync(kFullMask, q.x != 0u)) {
       const int dl = l - below, du = above - l;
       uint32_t lower = (uint32_t)(dl * dl) * 1024u + (uint32_t)(2 * y), up = (uint32_t)(2 * dl + 1) * 1024u;
       uint32_t upper = (uint32_t)(du * du) * 1024u + (uint32_t)(2 * y + 1), down = (uint32_t)(1 - 2 * du) * 1024u;
@@ -394,18 +409,32 @@ __device__ __forceinline__ void item_y(uint32_t* smem, const uint32_t* __restric
         k[i] = min(lower + up * i + (uint32_t)(i * (i - 1)) * 1024u, upper + down * i + (uint32_t)(i * (i - 1)) * 1024u);
       }
     } else {
+      // the chunk's own sites: the nearest outside these four z, then the distances step by step
+      const uint32_t lo = q.x & ((1u << l) - 1u), hi = (q.x >> l) >> 4, four = (q.x >> l) & 15u;
+      if (lo) below = 31 - __clz(lo);
+      if (hi) above = l + 3 + __ffs(hi);
+      int dl[4], du[4];
+      dl[0] = (four & 1u) ? 0 : l - below;
+      du[3] = above - l - 3;
+#pragma unroll
+      for (int i = 1; i < 4; ++i) {
+        dl[i] = (four >> i & 1u) ? 0 : dl[i - 1] + 1;
+        du[3 - i] = (four >> (4 - i) & 1u) ? 1 : du[4 - i] + 1;
+      }
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        const uint32_t le = (2u << (l + i)) - 1u, lo = q.x & le, hi = q.x & ~le;
-        const int b = lo ? 31 - __clz(lo) : below, a = hi ? __ffs(hi) - 1 : above;
-        const int dl = l + i - b, du = a - l - i, z = c * 32 + l + i;
-        uint32_t lower = (uint32_t)(dl * dl) * 1024u + (uint32_t)(2 * y);
-        if (Z > 512 && a == kNoneAbove && 1023 - z < dl) lower = kMissing;
-        k[i] = min(lower, (uint32_t)(du * du) * 1024u + (uint32_t)(2 * y + 1));
-        if (z >= Z) k[i] = kMissing;
+        uint32_t lower = (uint32_t)(dl[i] * dl[i]) * 1024u + (uint32_t)(2 * y);
+        const uint32_t upper = (uint32_t)(du[i] * du[i]) * 1024u + (uint32_t)(2 * y + 1);
+        if (Z > 512 && upper >= kMissing && 1023 - z0 - i < dl[i]) lower = kMissing;
+        k[i] = min(lower, upper);
       }
     }
-    *keys = make_uint4(k[0], k[1], k[2], k[3]);
+    if (c * 32 + 32 > Z) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (z0 + i >= Z) k[i] = kMissing;
+    }
+    if (y0 + (lane >> 3) < Y) *keys = make_uint4(k[0], k[1], k[2], k[3]);
   }
   OutY out{field + ((uint64_t)c * Y * X + x) * 32 + lane, X, Y};
   search_rows(s, out);
@@ -442,7 +471,8 @@ struct OutX {
   bool vec, none;
   uint32_t mask;        // row bits of a key, 0 where the column has no site
   uint32_t key[8], v[8];
-  int r = -1, rows_of;  // the pending rows: the first, and how many share key[0] (8 or 16; 1: eight keys)
+  int r = -1;           // first of the eight pending rows
+  bool one;             // they share key[0]
 
   __device__ __forceinline__ void begin(bool no_site) {
     none = no_site;
@@ -455,18 +485,12 @@ struct OutX {
   __device__ __forceinline__ void rows(int r_new, const uint32_t (&k)[8], bool same) {
     if (r >= 0) put();
     r = r_new;
-    rows_of = same ? 8 : 1;
+    one = same;
     fetch(0, k[0]);
     if (!same) {
 #pragma unroll
       for (int i = 1; i < 8; ++i) fetch(i, k[i]);
     }
-  }
-  __device__ __forceinline__ void same16(int r_new, uint32_t k, int) {
-    if (r >= 0) put();
-    r = r_new;
-    rows_of = 16;
-    fetch(0, k);
   }
   __device__ __forceinline__ uint32_t word(int i) const {
     const uint32_t y2s = v[i] & kRowBits;
@@ -477,34 +501,10 @@ struct OutX {
     const uint32_t zs = __float_as_uint(__fmaf_rn(dz2, half, zf));   // z in the low bits
     return none ? kDvUninit : (zs << 20) + ((y2s * 1024u + key[i]) >> 1);
   }
-  __device__ __forceinline__ void put16() {
-    const int lane = threadIdx.x & 31;
-    const uint32_t w = word(0);
-    if (vec && r + 16 <= X) {
-      uint32_t* p = dst + (uint64_t)((uint32_t)(lane >> 2) * layer + (uint32_t)(r + (lane & 3) * 4));
-#pragma unroll
-      for (int t = 0; t < 4; ++t, p += (uint64_t)layer * 8) {
-        const uint32_t o = __shfl_sync(kFullMask, w, t * 8 + (lane >> 2));
-        if (t * 8 + (lane >> 2) < z_rows) *reinterpret_cast<uint4*>(p) = make_uint4(o, o, o, o);
-      }
-    } else {
-      const int x = r + (lane & 15);
-      uint32_t* p = dst + (uint64_t)((uint32_t)(lane >> 4) * layer + (uint32_t)x);
-#pragma unroll 4
-      for (int z = lane >> 4; z < 32; z += 2, p += (uint64_t)layer * 2) {
-        const uint32_t o = __shfl_sync(kFullMask, w, z);
-        if (x < X && z < z_rows) *p = o;
-      }
-    }
-  }
   __device__ __forceinline__ void put() {
-    if (rows_of == 16) {
-      put16();
-      return;
-    }
     uint32_t w[8];
     w[0] = word(0);
-    if (rows_of == 8) {
+    if (one) {
 #pragma unroll
       for (int i = 1; i < 8; ++i) w[i] = w[0];
     } else {
@@ -550,6 +550,7 @@ __device__ __forceinline__ void item_x(uint32_t* smem, const uint32_t* __restric
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t* extra;
   const Search s = search_setup(smem, X, &extra);
+  wait_for_previous();
   const uint32_t* src = field + ((uint64_t)c * Y + y) * X * 32 + lane;
   // The item's rows are one piece of `field`: copied to the keys' place 16
   // bytes at a time, then a key's row bits (pass Y's row and side) replaced by x.
@@ -591,7 +592,10 @@ __global__ void __launch_bounds__(kWarps * 32, 3)
     search_y_kernel(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ near, uint32_t* __restrict__ field, int X,
                     int Y, int Z, const uint32_t* __restrict__ skip) {
   extern __shared__ __align__(16) uint32_t s_rows[];
-  if (skip != nullptr && *skip != 0u) return;
+  if (skip != nullptr) {
+    wait_for_previous();
+    if (*skip != 0u) return;
+  }
   item_y(s_rows, bits, near, field, X, Y, Z, blockIdx.x, blockIdx.y);
 }
 
@@ -599,7 +603,10 @@ __global__ void __launch_bounds__(kWarps * 32, 3)
     search_x_kernel(const uint32_t* __restrict__ field, uint32_t* __restrict__ map, int X, int Y, int Z,
                     const uint32_t* __restrict__ skip) {
   extern __shared__ __align__(16) uint32_t s_rows[];
-  if (skip != nullptr && *skip != 0u) return;
+  if (skip != nullptr) {
+    wait_for_previous();
+    if (*skip != 0u) return;
+  }
   item_x(s_rows, field, map, X, Y, Z, blockIdx.x, blockIdx.y);
 }
 
@@ -644,6 +651,7 @@ __device__ __forceinline__ void near_column(const uint32_t* __restrict__ bits, u
 template <int kMaxChunks>
 __global__ void __launch_bounds__(256) near_kernel(const uint32_t* __restrict__ bits, uint32_t* __restrict__ near,
                                                    uint32_t layer, int chunks, const uint32_t* __restrict__ skip) {
+  wait_for_previous();
   if (skip != nullptr && *skip != 0u) return;
   const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f < layer) near_column<kMaxChunks>(bits, near, layer, chunks, f);
@@ -759,6 +767,7 @@ __global__ void __launch_bounds__(256) zbits_from_map_batch_kernel(const BatchMa
 template <int kMaxChunks>
 __global__ void __launch_bounds__(256) near_batch_kernel(const BatchMap* __restrict__ maps, int skip_other) {
   const BatchMap m = maps[blockIdx.y];
+  wait_for_previous();
   if (skip_other && *other_flag(m) != 0u) return;
   const Areas a = areas(m);
   const uint32_t layer = (uint32_t)m.X * (uint32_t)m.Y;
@@ -772,7 +781,10 @@ __global__ void __launch_bounds__(kWarps * 32, 3)
   extern __shared__ __align__(16) uint32_t s_rows[];
   const uint32_t k = owner(prefix, n_maps, (long long)blockIdx.x);
   const BatchMap m = maps[k];
-  if (skip_other && *other_flag(m) != 0u) return;
+  if (skip_other) {
+    wait_for_previous();
+    if (*other_flag(m) != 0u) return;
+  }
   const int item = (int)((long long)blockIdx.x - __ldg(prefix + k)), c = item / m.X;
   const Areas a = areas(m);
   item_y(s_rows, a.bits, a.near, a.field, m.X, m.Y, m.Z, item - c * m.X, c);
@@ -784,7 +796,10 @@ __global__ void __launch_bounds__(kWarps * 32, 3)
   extern __shared__ __align__(16) uint32_t s_rows[];
   const uint32_t k = owner(prefix, n_maps, (long long)blockIdx.x);
   const BatchMap m = maps[k];
-  if (skip_other && *other_flag(m) != 0u) return;
+  if (skip_other) {
+    wait_for_previous();
+    if (*other_flag(m) != 0u) return;
+  }
   const int item = (int)((long long)blockIdx.x - __ldg(prefix + k)), c = item / m.Y;
   item_x(s_rows, areas(m).field, m.vox, m.X, m.Y, m.Z, item - c * m.Y, c);
 }
@@ -811,20 +826,34 @@ cudaError_t search_setup_once() {
   return err[dev];
 }
 
+// A launch that may begin while the kernel before it in the stream drains (it
+// calls wait_for_previous).
+template <class... P, class... A>
+cudaError_t launch_next(void (*kernel)(P...), dim3 grid, int smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute attr;
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(kWarps * 32);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = s;
+  cfg.attrs = &attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+
 // near, pass Y and pass X from the occupancy bits.
 cudaError_t launch_from_bits(uint32_t* map, const Areas& a, gvx_dims d, const uint32_t* skip, cudaStream_t s) {
   cudaError_t e = search_setup_once();
   if (e != cudaSuccess) return e;
   const int X = (int)d.x, Y = (int)d.y, Z = (int)d.z, zw = z_chunks(Z);
   const uint32_t layer = d.x * d.y;
-  const unsigned blocks = (layer + 255) / 256;
-  if (zw <= 4) near_kernel<4><<<blocks, 256, 0, s>>>(a.bits, a.near, layer, zw, skip);
-  else if (zw <= 8) near_kernel<8><<<blocks, 256, 0, s>>>(a.bits, a.near, layer, zw, skip);
-  else if (zw <= 16) near_kernel<16><<<blocks, 256, 0, s>>>(a.bits, a.near, layer, zw, skip);
-  else near_kernel<32><<<blocks, 256, 0, s>>>(a.bits, a.near, layer, zw, skip);
-  search_y_kernel<<<dim3(X, zw), kWarps * 32, smem_y(Y), s>>>(a.bits, a.near, a.field, X, Y, Z, skip);
-  search_x_kernel<<<dim3(Y, zw), kWarps * 32, smem_x(X), s>>>(a.field, map, X, Y, Z, skip);
-  return cudaGetLastError();
+  const auto near = zw <= 4 ? near_kernel<4> : zw <= 8 ? near_kernel<8> : zw <= 16 ? near_kernel<16> : near_kernel<32>;
+  e = launch_next(near, dim3((layer + 255) / 256), 0, s, a.bits, a.near, layer, zw, skip);
+  if (e == cudaSuccess) e = launch_next(search_y_kernel, dim3(X, zw), smem_y(Y), s, a.bits, a.near, a.field, X, Y, Z, skip);
+  if (e == cudaSuccess) e = launch_next(search_x_kernel, dim3(Y, zw), smem_x(X), s, a.field, map, X, Y, Z, skip);
+  return e;
 }
 
 }  // namespace
@@ -871,16 +900,18 @@ cudaError_t launch_from_bits_batch(const BatchMap* d_table, const BatchItems& it
   cudaError_t e = search_setup_once();
   if (e != cudaSuccess) return e;
   const int zw = z_chunks((int)it.z_max);
-  const dim3 grid(64, it.n_maps);
-  if (zw <= 4) near_batch_kernel<4><<<grid, 256, 0, s>>>(d_table, skip_other);
-  else if (zw <= 8) near_batch_kernel<8><<<grid, 256, 0, s>>>(d_table, skip_other);
-  else if (zw <= 16) near_batch_kernel<16><<<grid, 256, 0, s>>>(d_table, skip_other);
-  else near_batch_kernel<32><<<grid, 256, 0, s>>>(d_table, skip_other);
-  search_y_batch_kernel<<<(unsigned)it.total[4], kWarps * 32, smem_y((int)it.y_max), s>>>(d_table, it.d_prefix[4], it.n_maps,
-                                                                                          skip_other);
-  search_x_batch_kernel<<<(unsigned)it.total[5], kWarps * 32, smem_x((int)it.x_max), s>>>(d_table, it.d_prefix[5], it.n_maps,
-                                                                                          skip_other);
-  return cudaGetLastError();
+  const auto near = zw <= 4    ? near_batch_kernel<4>
+                    : zw <= 8  ? near_batch_kernel<8>
+                    : zw <= 16 ? near_batch_kernel<16>
+                               : near_batch_kernel<32>;
+  e = launch_next(near, dim3(64, it.n_maps), 0, s, d_table, skip_other);
+  if (e == cudaSuccess)
+    e = launch_next(search_y_batch_kernel, dim3((unsigned)it.total[4]), smem_y((int)it.y_max), s, d_table, it.d_prefix[4],
+                    it.n_maps, skip_other);
+  if (e == cudaSuccess)
+    e = launch_next(search_x_batch_kernel, dim3((unsigned)it.total[5]), smem_x((int)it.x_max), s, d_table, it.d_prefix[5],
+                    it.n_maps, skip_other);
+  return e;
 }
 }  // namespace
 
