@@ -1461,8 +1461,10 @@ cudaError_t launch_sweep_yx(uint32_t* map, uint32_t* scratch, uint64_t scratch_w
   blocks = sweep_blocks(blocks, scratch_words - sync_words(d), d, Cfg::kWarps, items);
   if (blocks < 1) return cudaErrorInvalidValue;
   unsigned* sync = scratch;
-  e = cudaMemsetAsync(sync, 0, (d.z + 2) * sizeof(unsigned), s);
-  if (e != cudaSuccess) return e;
+  if (run_if == nullptr) {  // launch_edt has cleared them before the flagged launch
+    e = cudaMemsetAsync(sync, 0, (d.z + 2) * sizeof(unsigned), s);
+    if (e != cudaSuccess) return e;
+  }
   edt_sweep_yx<kRows><<<(unsigned)blocks, Cfg::kWarps * 32, smem, s>>>(map, scratch + sync_words(d), sync, (int)d.x,
                                                                        (int)d.y, (int)d.z, run_if);
   return cudaGetLastError();

@@ -659,47 +659,41 @@ __global__ void __launch_bounds__(256) near_kernel(const uint32_t* __restrict__ 
 
 // Occupancy bits of a filled map.  A voxel holding another site than its own
 // sets *other_sites: the sweeps of edt.cu take the map then.  A block reads 32
-// x by 32 y columns of one chunk (a warp 4 of the y, a lane one x) and
-// stores the words with y fastest through shared memory.
+// x by 8 y columns of one chunk (a warp one y, a lane one x, 32 loads in
+// flight) and stores the words with y fastest through shared memory.  With 32
+// y per block 320 x 320 x 96 made 300 blocks, two per SM (13.8 us, now 9.2).
+constexpr int kTileY = 8;
 __device__ __forceinline__ bool zbits_tile(const uint32_t* __restrict__ map, uint32_t* __restrict__ bits, int X, int Y, int Z,
-                                           int bx, int by, int bz, uint32_t (&tile)[32][33]) {
+                                           int bx, int by, int bz, uint32_t (&tile)[kTileY][33]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int x = bx * 32 + lane, y0 = by * 32, z0 = bz * 32;
+  const int x = bx * 32 + lane, y = by * kTileY + warp, z0 = bz * 32;
   const uint64_t layer = (uint64_t)X * Y;
   bool other = false;
+  uint32_t word = 0u;
+  if (x < X && y < Y) {
+    const uint32_t* src = map + (uint64_t)z0 * layer + (uint64_t)y * X + x;
+    const uint32_t own = (uint32_t)x | (uint32_t)y << 10 | (uint32_t)z0 << 20;
+    uint32_t v[32];
 #pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int y = y0 + warp * 4 + k;
-    uint32_t word = 0u;
-    if (x < X && y < Y) {
-      const uint32_t* src = map + (uint64_t)z0 * layer + (uint64_t)y * X + x;
-      const uint32_t own = (uint32_t)x | (uint32_t)y << 10 | (uint32_t)z0 << 20;
-      uint32_t v[32];
+    for (int i = 0; i < 32; ++i) v[i] = z0 + i < Z ? __ldg(src + (uint64_t)i * layer) : kDvUninit;
 #pragma unroll
-      for (int i = 0; i < 32; ++i) v[i] = z0 + i < Z ? __ldg(src + (uint64_t)i * layer) : kDvUninit;
-#pragma unroll
-      for (int i = 0; i < 32; ++i) {
-        if (v[i] != kDvUninit) {
-          word |= 1u << i;
-          other |= v[i] != own + ((uint32_t)i << 20);
-        }
+    for (int i = 0; i < 32; ++i) {
+      if (v[i] != kDvUninit) {
+        word |= 1u << i;
+        other |= v[i] != own + ((uint32_t)i << 20);
       }
     }
-    tile[warp * 4 + k][lane] = word;
   }
+  tile[warp][lane] = word;
   __syncthreads();
-  const int y = y0 + lane;
-#pragma unroll
-  for (int k = 0; k < 4; ++k) {
-    const int xo = bx * 32 + warp * 4 + k;
-    if (xo < X && y < Y) bits[((uint64_t)bz * X + xo) * Y + y] = tile[lane][warp * 4 + k];
-  }
+  const int xo = bx * 32 + (threadIdx.x >> 3), yo = by * kTileY + (threadIdx.x & 7);
+  if (xo < X && yo < Y) bits[((uint64_t)bz * X + xo) * Y + yo] = tile[threadIdx.x & 7][threadIdx.x >> 3];
   return other;
 }
 
 __global__ void __launch_bounds__(256) zbits_from_map_kernel(const uint32_t* __restrict__ map, uint32_t* __restrict__ bits,
                                                              int X, int Y, int Z, uint32_t* __restrict__ other_sites) {
-  __shared__ uint32_t tile[32][33];
+  __shared__ uint32_t tile[kTileY][33];
   const bool other = zbits_tile(map, bits, X, Y, Z, blockIdx.x, blockIdx.y, blockIdx.z, tile);
   if (__any_sync(kFullMask, other) && (threadIdx.x & 31) == 0) atomicOr(other_sites, 1u);
 }
@@ -752,10 +746,10 @@ __global__ void zbits_insert_batch_kernel(const BatchMap* __restrict__ maps, uin
 
 // block row = map; the blocks of a row stride over the map's tiles
 __global__ void __launch_bounds__(256) zbits_from_map_batch_kernel(const BatchMap* __restrict__ maps) {
-  __shared__ uint32_t tile[32][33];
+  __shared__ uint32_t tile[kTileY][33];
   const BatchMap m = maps[blockIdx.y];
   uint32_t* bits = areas(m).bits;
-  const int tx = (m.X + 31) >> 5, ty = (m.Y + 31) >> 5, tiles = tx * ty * z_chunks(m.Z);
+  const int tx = (m.X + 31) >> 5, ty = (m.Y + kTileY - 1) / kTileY, tiles = tx * ty * z_chunks(m.Z);
   bool other = false;
   for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
     other |= zbits_tile(m.vox, bits, m.X, m.Y, m.Z, t % tx, t / tx % ty, t / (tx * ty), tile);
@@ -885,7 +879,7 @@ cudaError_t launch_search_voxelize(uint32_t* d_vox, uint32_t* area, gvx_dims d, 
 
 cudaError_t launch_search_filled(uint32_t* d_vox, uint32_t* area, gvx_dims d, uint32_t* d_other, cudaStream_t s) {
   const Areas a = areas(area, (int)d.x, (int)d.y, (int)d.z);
-  const dim3 grid((d.x + 31) / 32, (d.y + 31) / 32, (unsigned)z_chunks((int)d.z));
+  const dim3 grid((d.x + 31) / 32, (d.y + kTileY - 1) / kTileY, (unsigned)z_chunks((int)d.z));
   zbits_from_map_kernel<<<grid, 256, 0, s>>>(d_vox, a.bits, (int)d.x, (int)d.y, (int)d.z, d_other);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? launch_from_bits(d_vox, a, d, d_other, s) : e;

@@ -1,0 +1,27 @@
+"""ProbVoxelMap inserts whose neighbouring points share voxels and 4-voxel words (one swap per word and warp) against
+the oracle, which applies the points one by one."""
+import numpy as np
+import pytest
+import torch
+
+import gvx
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("n", [1, 31, 32, 33, 1000, 40_000])
+@pytest.mark.parametrize("spread", [3, 60, 100_000])
+def test_runs_of_points(n, spread):
+    dims = (37, 29, 23)
+    rng = np.random.default_rng(n + spread)
+    g, o = gvx.ProbVoxelMap(dims, 1.0), oracle.pvm_empty(dims)
+    for meaning in (1, 0, 129, 90, 254, 0, 4, 255, 2):
+        ids = np.sort(rng.integers(0, min(spread, dims[0] * dims[1] * dims[2]), n))
+        pts = np.stack([ids % dims[0], ids // dims[0] % dims[1], ids // (dims[0] * dims[1])], 1) + 0.5
+        pts[rng.random(n) < 0.05] = -3e9  # the reference's saturating conversion puts these into voxel 0
+        pts[rng.random(n) < 0.05] = 1e9  # outside
+        pts = pts.astype(np.float32)
+        g.insertPointCloud(torch.as_tensor(pts), meaning)
+        oracle.pvm_insert(o, dims, 1.0, pts, meaning)
+        assert np.array_equal(g.data().cpu().numpy(), o)
