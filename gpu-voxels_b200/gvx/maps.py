@@ -255,26 +255,27 @@ class DistanceVoxelMap:
         return out
 
 
+class _DeviceBuffer:
+    """A raw device pointer in the form torch borrows it in.  (Defined once: a
+    class made for each view cost more than the view.)"""
+
+    __slots__ = ("__cuda_array_interface__",)
+
+    def __init__(self, ptr: int, n: int, typestr: str):
+        self.__cuda_array_interface__ = {"shape": (n,), "typestr": typestr, "data": (ptr, False), "version": 3}
+
+
 def _device_view(ptr: int, n: int) -> torch.Tensor:
     """A borrowed int32 CUDA tensor over n elements at a raw device pointer."""
-    class _CAI:
-        __cuda_array_interface__ = {"shape": (n,), "typestr": "<i4", "data": (ptr, False), "version": 3}
-
-    return torch.as_tensor(_CAI(), device="cuda")
+    return torch.as_tensor(_DeviceBuffer(ptr, n, "<i4"), device="cuda")
 
 
 def _device_view_u8(ptr: int, n: int) -> torch.Tensor:
-    class _CAI:
-        __cuda_array_interface__ = {"shape": (n,), "typestr": "|u1", "data": (ptr, False), "version": 3}
-
-    return torch.as_tensor(_CAI(), device="cuda")
+    return torch.as_tensor(_DeviceBuffer(ptr, n, "|u1"), device="cuda")
 
 
 def _device_view_i8(ptr: int, n: int) -> torch.Tensor:
-    class _CAI:
-        __cuda_array_interface__ = {"shape": (n,), "typestr": "|i1", "data": (ptr, False), "version": 3}
-
-    return torch.as_tensor(_CAI(), device="cuda")
+    return torch.as_tensor(_DeviceBuffer(ptr, n, "|i1"), device="cuda")
 
 
 def extract_given_distances(dist_map: "DistanceVoxelMap", min_dist: int, max_dist: int,
