@@ -298,50 +298,71 @@ __global__ void __launch_bounds__(256) lists_collide_bits_kernel(const uint32_t*
   }
   // Entry e of lane l in group g is g * kG + e * 32 + l: each load covers 32
   // consecutive entries of a sorted list, so its bit lookups fall in few lines.
-  auto load_ids = [&](uint64_t g, uint32_t (&j)[kE]) {
-    const uint64_t k0 = g * kG + (uint64_t)lane;
+  // The loop is bound by instruction issue: entries are counted down in 32
+  // bits from the warp's first one, a whole group is loaded without a check per
+  // entry, and one vote tells whether any of its 128 entries is a candidate
+  // (37 instructions per 32 entries before, most of them 64-bit index checks).
+  const uint32_t in_map = (uint32_t)min(map_n, (uint64_t)0xFFFFFFFFu);
+  const uint32_t* idp = ids + g_begin * kG + lane;
+  int64_t left = (int64_t)(min(n_total, g_end * kG) - g_begin * kG) - lane;  // this lane's entries are e * 32 < left
+  uint64_t k0 = g_begin * kG + (uint64_t)lane;
+  auto load_ids = [&](const uint32_t* p, int64_t n, uint32_t (&j)[kE]) {
+    if (n > (kE - 1) * 32) {
 #pragma unroll
-    for (int e = 0; e < kE; ++e) j[e] = (g < g_end && k0 + e * 32 < n_total) ? __ldg(ids + k0 + e * 32) : 0xFFFFFFFFu;
+      for (int e = 0; e < kE; ++e) j[e] = __ldg(p + e * 32);
+    } else {
+#pragma unroll
+      for (int e = 0; e < kE; ++e) j[e] = e * 32 < n ? __ldg(p + e * 32) : 0xFFFFFFFFu;
+    }
   };
   int queued = 0;  // warp-uniform
   uint32_t jn[kE];
-  load_ids(g_begin, jn);
-  for (uint64_t g = g_begin; g < g_end; ++g) {
-    uint32_t j[kE];
-#pragma unroll
-    for (int e = 0; e < kE; ++e) j[e] = jn[e];
-    load_ids(g + 1, jn);  // the next group's ids in flight while this one is tested
-    unsigned occ = 0;
-#pragma unroll
-    for (int e = 0; e < kE; ++e)
-      occ |= (unsigned)(j[e] < map_n && ((__ldg(bits + (j[e] >> 5)) >> (j[e] & 31)) & 1u)) << e;
-    const uint64_t k0 = g * kG + (uint64_t)lane;
+  load_ids(idp, left, jn);
+  const uint64_t k_end = min(n_total, g_end * kG);  // warp-uniform end of the range
+  for (uint64_t kg = g_begin * kG; kg < k_end; kg += kG, k0 += kG) {
+    uint32_t j[kE], w[kE];
 #pragma unroll
     for (int e = 0; e < kE; ++e) {
-      const bool c = (occ >> e) & 1u;
-      const unsigned cm = __ballot_sync(kFull, c);
-      if (cm) {  // append this round's candidates to the queue
-        if (c) {
-          const int slot = queued + __popc(cm & ((1u << lane) - 1u));
-          cand_k[slot] = k0 + e * 32;
-          cand_lb[slot] = list;
-        }
-        queued += __popc(cm);
-        __syncwarp();
-        if (queued >= 32) {
-          flush_candidates(cand_k, cand_lb, 32, lvox, offsets, n_lists, mark, counts);
-          __syncwarp();
-          queued -= 32;
-          if (lane < queued) {  // the remainder moves to the front
-            cand_k[lane] = cand_k[32 + lane];
-            cand_lb[lane] = cand_lb[32 + lane];
+      j[e] = jn[e];
+      w[e] = j[e] < in_map ? __ldg(bits + (j[e] >> 5)) : 0u;
+    }
+    idp += kG;
+    left -= kG;
+    load_ids(idp, left, jn);  // the next group's ids in flight while this one is tested
+    uint32_t any = 0u;
+#pragma unroll
+    for (int e = 0; e < kE; ++e) {
+      w[e] = __funnelshift_r(w[e], 0u, j[e]);  // the entry's bit to bit 0
+      any |= w[e];
+    }
+    if (__any_sync(kFull, any & 1u)) {
+#pragma unroll
+      for (int e = 0; e < kE; ++e) {
+        const bool c = w[e] & 1u;
+        const unsigned cm = __ballot_sync(kFull, c);
+        if (cm) {  // append this round's candidates to the queue
+          if (c) {
+            const int slot = queued + __popc(cm & ((1u << lane) - 1u));
+            cand_k[slot] = k0 + e * 32;
+            cand_lb[slot] = list;
           }
+          queued += __popc(cm);
           __syncwarp();
+          if (queued >= 32) {
+            flush_candidates(cand_k, cand_lb, 32, lvox, offsets, n_lists, mark, counts);
+            __syncwarp();
+            queued -= 32;
+            if (lane < queued) {  // the remainder moves to the front
+              cand_k[lane] = cand_k[32 + lane];
+              cand_lb[lane] = cand_lb[32 + lane];
+            }
+            __syncwarp();
+          }
         }
       }
     }
     // the bound for the next group: the list of its first entry
-    const uint64_t next = min((g + 1) * kG, n_total - 1);
+    const uint64_t next = min(kg + kG, n_total - 1);
     while (list + 1 < n_lists && __ldg(offsets + list + 1) <= next) ++list;
   }
   if (queued > 0) flush_candidates(cand_k, cand_lb, queued, lvox, offsets, n_lists, mark, counts);
