@@ -34,10 +34,10 @@
 // What bounds it: instruction issue and the 2-cycle integer pipe (65 % and 70 %
 // busy; a candidate costs one add-and-min, no divide, no per-lane control
 // flow); DRAM is a third busy.  Measured on a B200 against the sweeps of edt.cu
-// (whole calls, warm): 512^3 depth scene 810 us against 1710 (pass Y 358, pass X
-// 440); 128^3 with 50k box points 37 against 183 (the sweeps walk 128 rows one
+// (whole calls, warm): 512^3 depth scene 798 us against 1710 (pass Y 344, pass X
+// 426); 128^3 with 50k box points 36 against 183 (the sweeps walk 128 rows one
 // after another per pass, here 8 warps share a column); 203 x 331 x 157 in three
-// calls 145 against 491; 24 uneven maps of 64 to 384 per axis in one batch 1551
+// calls 139 against 491; 24 uneven maps of 64 to 384 per axis in one batch 1499
 // against 2606.
 //
 // The searching loops are kept rolled: unrolled over a warp's rows the code
@@ -96,6 +96,22 @@ __host__ __device__ __forceinline__ int search_smem_words(int L, int extra) {
   return key_rows(L) * 32 + weight_words(L) + kWarps * 32 + least_words(L) + extra;
 }
 
+// 1024 d^2 for d = -511 .. 512, copied into every block's shared memory (16
+// bytes a copy; computing them took 40 instructions of each warp).
+struct WeightTable {
+  uint32_t w[2 * kMaxLen];
+  constexpr WeightTable() : w() {
+    for (int i = 0; i < 2 * kMaxLen; ++i) w[i] = (uint32_t)((i - kMaxLen + 1) * (i - kMaxLen + 1)) << 10;
+  }
+};
+__device__ const __align__(16) WeightTable g_weights{};
+
+__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
+  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem_src) : "memory");
+}
+__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
+
 struct Search {
   uint32_t* key;      // this lane's column: key[row * 32]
   const uint32_t* w;  // weight of offset d at w[d]; w[d - 3] is 16-byte aligned for d a multiple of 4
@@ -104,14 +120,17 @@ struct Search {
   int L;
 };
 
+// The block's tables; the weights arrive with the caller's cp_async_wait_all
+// and barrier.
 __device__ __forceinline__ Search search_setup(uint32_t* smem, int L, uint32_t** extra) {
   const int lane = threadIdx.x & 31;
   Search s;
   s.L = L;
   s.key = smem + lane;
   uint32_t* w = smem + key_rows(L) * 32;
-  const int off = kWarps * seg_rows(L) - 1;
-  for (int i = threadIdx.x; i < weight_words(L); i += kWarps * 32) w[i] = (uint32_t)((i - off) * (i - off)) << 10;
+  const int off = kWarps * seg_rows(L) - 1;  // the word of d = 0; the table's starts at kMaxLen - 1
+  for (int i = threadIdx.x; i < weight_words(L) / 4; i += kWarps * 32)
+    cp_async16(w + 4 * i, g_weights.w + (kMaxLen - 1 - off) + 4 * i);
   s.w = w + off;
   uint32_t* bnd = w + weight_words(L);
   bnd[threadIdx.x] = 0xffffffffu;
@@ -268,8 +287,17 @@ __device__ __forceinline__ void segment_starts(const Search& s, int warp, int S,
   if (seg0 < s.L) {
     const bool some = least < kNoSite;
     least &= ~1023u;
+    // the worst of all starts against the nearest any of them can be: mostly
+    // nothing is left to look at one by one
+    uint32_t worst = 0u;
+#pragma unroll
+    for (int i = 0; i < kWarps; ++i) {
+      const uint32_t have = *reinterpret_cast<volatile uint32_t*>(s.bnd + i * 32);
+      if (i != warp && i != warp + 1 && i * S < s.L) worst = max(worst, have);
+    }
+    const bool look = __any_sync(kFullMask, some && least + s.w[S] <= worst);
 #pragma unroll 1
-    for (int i = 0; i < kWarps && i * S < s.L; ++i) {
+    for (int i = 0; look && i < kWarps && i * S < s.L; ++i) {
       if (i == warp || i == warp + 1) continue;
       const int gap = i < warp ? seg0 - i * S : i * S - (seg1 - 1);
       // a start's key only ever falls: a stale one only lets the scan run
@@ -360,15 +388,23 @@ __device__ __forceinline__ void search_rows(const Search& s, Out& out) {
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void start_next() { asm volatile("griddepcontrol.launch_dependents;"); }
 
+// Pass Y's rows into `field`, byte offsets in 32 bits (512 x 512 x 1023: 1.1 GB).
 struct OutY {
-  uint32_t* out;  // row 0 of this lane's column in `field`
-  int X, Y;
+  uint32_t* field;
+  uint32_t first, row_bytes;  // of this lane's row 0; from a row to the next
+  int Y;
   __device__ __forceinline__ void begin(bool) {}
   __device__ __forceinline__ void rows(int r, const uint32_t (&k)[8], bool) {
-    uint32_t* o = out + (uint32_t)(r * X) * 32u;
+    char* base = reinterpret_cast<char*>(field);
+    uint32_t at = first + (uint32_t)r * row_bytes;
+    if (r + 8 <= Y) {
 #pragma unroll
-    for (int i = 0; i < 8; ++i, o += (uint32_t)X * 32u)
-      if (r + i < Y) *o = k[i];
+      for (int i = 0; i < 8; ++i, at += row_bytes) *reinterpret_cast<uint32_t*>(base + at) = k[i];
+    } else {
+#pragma unroll
+      for (int i = 0; i < 8; ++i, at += row_bytes)
+        if (r + i < Y) *reinterpret_cast<uint32_t*>(base + at) = k[i];
+    }
   }
   __device__ __forceinline__ void finish() {}
 };
@@ -384,67 +420,66 @@ __device__ __forceinline__ void item_y(uint32_t* smem, const uint32_t* __restric
   uint2* col = reinterpret_cast<uint2*>(extra);  // (bits, near) of every y
   const uint64_t base = ((uint64_t)c * X + x) * Y;
   for (int y = threadIdx.x; y < Y; y += kWarps * 32) col[y] = make_uint2(__ldg(bits + base + y), __ldg(near + base + y));
+  cp_async_wait_all();
   __syncthreads();
   // The nearest site of the (x, y) column by phase 1's rule
   // (kernelPBAphase1FloodZ, GV/voxelmap/kernels/VoxelMapOperationsPBA.hpp:63-124):
   // the lower of two equally near ones.  Without a site above the reference
   // puts one at 1023, and where that is nearer the voxel stays uninitialised
-  // (only possible when Z is above 512).  A thread makes the keys of 4
-  // consecutive z: where the chunk holds no site of the column, a square's
-  // step to the next z is one addition.
-  const int l = 4 * (threadIdx.x & 7), z0 = c * 32 + l;
-  uint4* keys = reinterpret_cast<uint4*>(smem) + threadIdx.x;
+  // (only possible when Z is above 512).
+  // Four lanes make the 32 keys of one y, two quads of z each (odd y the upper
+  // quad first: no bank conflicts).
 #pragma unroll 1
-  for (int y0 = (threadIdx.x >> 5) * 4; y0 < Y; y0 += kWarps * 4, keys += kWarps * 32) {  // four y per warp
-    const int y = min(y0 + (lane >> 3), Y - 1);
+  for (int y0 = (threadIdx.x >> 5) * 8; y0 < Y; y0 += kWarps * 8) {  // eight y per warp
+    const int y = min(y0 + (lane >> 2), Y - 1);
+    const bool store = y0 + (lane >> 2) < Y;
     const uint2 q = col[y];
-    int below = (int)(short)(q.y & 0xffffu), above = (int)q.y >> 16;
-    uint32_t k[4];
-    if (Z <= 512 && !__any_sync(kFullMask, q.x != 0u)) {
-      const int dl = l - below, du = above - l;
-      uint32_t lower = (uint32_t)(dl * dl) * 1024u + (uint32_t)(2 * y), up = (uint32_t)(2 * dl + 1) * 1024u;
-      uint32_t upper = (uint32_t)(du * du) * 1024u + (uint32_t)(2 * y + 1), down = (uint32_t)(1 - 2 * du) * 1024u;
+    const bool plain = Z <= 512 && !__any_sync(kFullMask, q.x != 0u);
+    uint4* keys = reinterpret_cast<uint4*>(smem) + y * 8;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        k[i] = min(lower + up * i + (uint32_t)(i * (i - 1)) * 1024u, upper + down * i + (uint32_t)(i * (i - 1)) * 1024u);
-      }
-    } else {
-      // the chunk's own sites: the nearest outside these four z, then the distances step by step
-      const uint32_t lo = q.x & ((1u << l) - 1u), hi = (q.x >> l) >> 4, four = (q.x >> l) & 15u;
-      if (lo) below = 31 - __clz(lo);
-      if (hi) above = l + 3 + __ffs(hi);
-      int dl[4], du[4];
-      dl[0] = (four & 1u) ? 0 : l - below;
-      du[3] = above - l - 3;
+    for (int half = 0; half < 2; ++half) {
+      const int quad = (lane & 3) + 4 * ((y ^ half) & 1), l = 4 * quad;
+      int below = (int)(short)(q.y & 0xffffu), above = (int)q.y >> 16;
+      uint32_t k[4];
+      if (plain) {
+        const int dl = 32 * (l - below), du = 32 * (above - l);
 #pragma unroll
-      for (int i = 1; i < 4; ++i) {
-        dl[i] = (four >> i & 1u) ? 0 : dl[i - 1] + 1;
-        du[3 - i] = (four >> (4 - i) & 1u) ? 1 : du[4 - i] + 1;
-      }
+        for (int i = 0; i < 4; ++i) {
+          const uint32_t a = (uint32_t)(dl + 32 * i), b = (uint32_t)(du - 32 * i);
+          k[i] = min(a * a + (uint32_t)(2 * y), b * b + (uint32_t)(2 * y + 1));
+        }
+      } else {
+        // the chunk's own sites: the nearest outside these four z, then the distances step by step
+        const uint32_t lo = q.x & ((1u << l) - 1u), hi = (q.x >> l) >> 4, four = (q.x >> l) & 15u;
+        if (lo) below = 31 - __clz(lo);
+        if (hi) above = l + 3 + __ffs(hi);
+        int dl[4], du[4];
+        dl[0] = (four & 1u) ? 0 : l - below;
+        du[3] = above - l - 3;
 #pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        uint32_t lower = (uint32_t)(dl[i] * dl[i]) * 1024u + (uint32_t)(2 * y);
-        const uint32_t upper = (uint32_t)(du[i] * du[i]) * 1024u + (uint32_t)(2 * y + 1);
-        if (Z > 512 && upper >= kMissing && 1023 - z0 - i < dl[i]) lower = kMissing;
-        k[i] = min(lower, upper);
+        for (int i = 1; i < 4; ++i) {
+          dl[i] = (four >> i & 1u) ? 0 : dl[i - 1] + 1;
+          du[3 - i] = (four >> (4 - i) & 1u) ? 1 : du[4 - i] + 1;
+        }
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint32_t lower = (uint32_t)(dl[i] * dl[i]) * 1024u + (uint32_t)(2 * y);
+          const uint32_t upper = (uint32_t)(du[i] * du[i]) * 1024u + (uint32_t)(2 * y + 1);
+          if (Z > 512 && upper >= kMissing && 1023 - (c * 32 + l + i) < dl[i]) lower = kMissing;
+          k[i] = min(lower, upper);
+        }
       }
+      if (c * 32 + 32 > Z) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (c * 32 + l + i >= Z) k[i] = kMissing;
+      }
+      if (store) keys[quad] = make_uint4(k[0], k[1], k[2], k[3]);
     }
-    if (c * 32 + 32 > Z) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-        if (z0 + i >= Z) k[i] = kMissing;
-    }
-    if (y0 + (lane >> 3) < Y) *keys = make_uint4(k[0], k[1], k[2], k[3]);
   }
-  OutY out{field + ((uint64_t)c * Y * X + x) * 32 + lane, X, Y};
+  OutY out{field, (((uint32_t)c * Y * X + x) * 32 + lane) * 4u, (uint32_t)X * 128u, Y};
   search_rows(s, out);
 }
-
-__device__ __forceinline__ void cp_async16(void* smem_dst, const void* gmem_src) {
-  const unsigned s = static_cast<unsigned>(__cvta_generic_to_shared(smem_dst));
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(s), "l"(gmem_src) : "memory");
-}
-__device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;\n" ::: "memory"); }
 
 __device__ __forceinline__ float sqrt_approx(float v) {
   float r;
@@ -584,11 +619,15 @@ __device__ __forceinline__ void item_x(uint32_t* smem, const uint32_t* __restric
   search_rows(s, out);
 }
 
+// Resident blocks the registers must allow: pass Y four (64 registers; four fit
+// the shared memory up to 384 rows, and 69 registers took three, 24 maps' pass
+// Y 682 us against 634), pass X three (at 64 registers it spills: 512^3 447 ->
+// 486 us).
 constexpr int kStageWords = kWarps * 128;
 int smem_y(int Y) { return search_smem_words(Y, 2 * Y) * 4; }
 int smem_x(int X) { return search_smem_words(X, kStageWords) * 4; }
 
-__global__ void __launch_bounds__(kWarps * 32, 3)
+__global__ void __launch_bounds__(kWarps * 32, 4)
     search_y_kernel(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ near, uint32_t* __restrict__ field, int X,
                     int Y, int Z, const uint32_t* __restrict__ skip) {
   extern __shared__ __align__(16) uint32_t s_rows[];
@@ -759,17 +798,26 @@ __global__ void __launch_bounds__(256) zbits_from_map_batch_kernel(const BatchMa
 }
 
 template <int kMaxChunks>
-__global__ void __launch_bounds__(256) near_batch_kernel(const BatchMap* __restrict__ maps, int skip_other) {
-  const BatchMap m = maps[blockIdx.y];
-  wait_for_previous();
-  if (skip_other && *other_flag(m) != 0u) return;
+__device__ __forceinline__ void near_map(const BatchMap& m) {
   const Areas a = areas(m);
   const uint32_t layer = (uint32_t)m.X * (uint32_t)m.Y;
   for (uint32_t f = blockIdx.x * blockDim.x + threadIdx.x; f < layer; f += gridDim.x * blockDim.x)
     near_column<kMaxChunks>(a.bits, a.near, layer, z_chunks(m.Z), f);
 }
 
-__global__ void __launch_bounds__(kWarps * 32, 3)
+// block row = map, each with the registers and loads of its own height
+__global__ void __launch_bounds__(256) near_batch_kernel(const BatchMap* __restrict__ maps, int skip_other) {
+  const BatchMap m = maps[blockIdx.y];
+  wait_for_previous();
+  if (skip_other && *other_flag(m) != 0u) return;
+  const int chunks = z_chunks(m.Z);
+  if (chunks <= 4) near_map<4>(m);
+  else if (chunks <= 8) near_map<8>(m);
+  else if (chunks <= 16) near_map<16>(m);
+  else near_map<32>(m);
+}
+
+__global__ void __launch_bounds__(kWarps * 32, 4)
     search_y_batch_kernel(const BatchMap* __restrict__ maps, const long long* __restrict__ prefix, uint32_t n_maps,
                           int skip_other) {
   extern __shared__ __align__(16) uint32_t s_rows[];
@@ -893,12 +941,7 @@ namespace {
 cudaError_t launch_from_bits_batch(const BatchMap* d_table, const BatchItems& it, int skip_other, cudaStream_t s) {
   cudaError_t e = search_setup_once();
   if (e != cudaSuccess) return e;
-  const int zw = z_chunks((int)it.z_max);
-  const auto near = zw <= 4    ? near_batch_kernel<4>
-                    : zw <= 8  ? near_batch_kernel<8>
-                    : zw <= 16 ? near_batch_kernel<16>
-                               : near_batch_kernel<32>;
-  e = launch_next(near, dim3(64, it.n_maps), 0, s, d_table, skip_other);
+  e = launch_next(near_batch_kernel, dim3(128, it.n_maps), 0, s, d_table, skip_other);
   if (e == cudaSuccess)
     e = launch_next(search_y_batch_kernel, dim3((unsigned)it.total[4]), smem_y((int)it.y_max), s, d_table, it.d_prefix[4],
                     it.n_maps, skip_other);
