@@ -66,12 +66,17 @@ __global__ void trilinear_bwd_kernel(MapView m, const float* __restrict__ xyz, u
 // F_j alone).  With one lane of a warp walking the whole chain of the warp's
 // configuration the rest of the warp idled through seven FP64 sincos and matrix
 // products: cost and adjoint of 512 trajectories x 64 waypoints x 56 spheres
-// through autograd took 306 us, now 146; 4096 clearances 22.5 us, now 13.4.
-// The rest is bound by the corner gathers and their arithmetic.
+// through autograd took 306 us, then 146; 4096 clearances 22.5 us, then 13.4.
+// The rest is bound by the queries' arithmetic (127 and 12.3 us with their packed form).
 // ---------------------------------------------------------------------------
 constexpr int kWarpsPerBlock = 8;
 constexpr int kThreads = kWarpsPerBlock * 32;
 constexpr int kMaxBlockConfigs = 64;
+// Blocks of an SM the clearance and cost kernels keep room for: four (64
+// registers) take 512 trajectories at once, where three (75 to 80 registers)
+// left a second wave (cost 52 us against 50, 4096 clearances 11.9 against 10.3).
+// The adjoint's FP64 sums spill at 64 and at 80 registers (91 us); left at 124 it takes 74.
+constexpr int kArmBlocks = 4;
 
 // Shared memory of a block for `configs` configurations.
 struct ArmSmem {
@@ -148,7 +153,7 @@ __device__ __forceinline__ void sphere_centre(const ArmSmem& a, const double* po
 }
 
 // Min clearance per configuration; one warp per configuration, lanes over spheres.
-__global__ void __launch_bounds__(kThreads) sphere_clearance_kernel(MapView m, gvx_arm arm, const float* __restrict__ q,
+__global__ void __launch_bounds__(kThreads, kArmBlocks) sphere_clearance_kernel(MapView m, gvx_arm arm, const float* __restrict__ q,
                                                                     uint64_t n_cfg, int per_block,
                                                                     float* __restrict__ out) {
   extern __shared__ __align__(16) double s_arm[];
@@ -178,7 +183,7 @@ __global__ void __launch_bounds__(kThreads) sphere_clearance_kernel(MapView m, g
 
 // Hinge cost: one block per trajectory, warp w takes waypoints w, w+8, ...;
 // fixed-order reductions keep the result deterministic.
-__global__ void __launch_bounds__(kThreads) traj_cost_kernel(MapView m, gvx_arm arm, const float* __restrict__ q,
+__global__ void __launch_bounds__(kThreads, kArmBlocks) traj_cost_kernel(MapView m, gvx_arm arm, const float* __restrict__ q,
                                                              uint64_t n_traj, uint32_t n_wp, int per_block, float margin,
                                                              float* __restrict__ cost) {
   extern __shared__ __align__(16) double s_arm[];
