@@ -388,6 +388,17 @@ __device__ __forceinline__ void search_rows(const Search& s, Out& out) {
 __device__ __forceinline__ void wait_for_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void start_next() { asm volatile("griddepcontrol.launch_dependents;"); }
 
+// A word that an earlier kernel of the chain writes.  That kernel may still run
+// when this one begins, so the word is not read-only for this kernel's lifetime:
+// no __ldg and no const __restrict__ parameter (either lets the compiler read
+// through the non-coherent path, and early).  Volatile keeps the load after
+// wait_for_previous.
+__device__ __forceinline__ uint32_t load_chained(const uint32_t* p) {
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
+
 // Pass Y's rows into `field`, byte offsets in 32 bits (512 x 512 x 1023: 1.1 GB).
 struct OutY {
   uint32_t* field;
@@ -410,8 +421,7 @@ struct OutY {
 };
 
 // Pass Y of plane x, chunk c: the nearest site in the (y, z) plane.
-__device__ __forceinline__ void item_y(uint32_t* smem, const uint32_t* __restrict__ bits, const uint32_t* __restrict__ near,
-                                       uint32_t* __restrict__ field, int X, int Y, int Z, int x, int c) {
+__device__ __forceinline__ void item_y(uint32_t* smem, const uint32_t* bits, const uint32_t* near, uint32_t* field, int X, int Y, int Z, int x, int c) {
   const int lane = threadIdx.x & 31;
   uint32_t* extra;
   const Search s = search_setup(smem, Y, &extra);
@@ -419,7 +429,7 @@ __device__ __forceinline__ void item_y(uint32_t* smem, const uint32_t* __restric
   wait_for_previous();
   uint2* col = reinterpret_cast<uint2*>(extra);  // (bits, near) of every y
   const uint64_t base = ((uint64_t)c * X + x) * Y;
-  for (int y = threadIdx.x; y < Y; y += kWarps * 32) col[y] = make_uint2(__ldg(bits + base + y), __ldg(near + base + y));
+  for (int y = threadIdx.x; y < Y; y += kWarps * 32) col[y] = make_uint2(load_chained(bits + base + y), load_chained(near + base + y));
   cp_async_wait_all();
   __syncthreads();
   // The nearest site of the (x, y) column by phase 1's rule
@@ -515,7 +525,7 @@ struct OutX {
   }
   __device__ __forceinline__ void fetch(int i, uint32_t k) {
     key[i] = k & mask;
-    v[i] = __ldg(src + key[i] * 16u);
+    v[i] = load_chained(src + key[i] * 16u);
   }
   __device__ __forceinline__ void rows(int r_new, const uint32_t (&k)[8], bool same) {
     if (r >= 0) put();
@@ -580,7 +590,7 @@ struct OutX {
 };
 
 // Pass X of plane y, chunk c: the nearest site of the map, written to the map.
-__device__ __forceinline__ void item_x(uint32_t* smem, const uint32_t* __restrict__ field, uint32_t* __restrict__ map, int X,
+__device__ __forceinline__ void item_x(uint32_t* smem, const uint32_t* field, uint32_t* map, int X,
                                        int Y, int Z, int y, int c) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   uint32_t* extra;
@@ -628,23 +638,21 @@ int smem_y(int Y) { return search_smem_words(Y, 2 * Y) * 4; }
 int smem_x(int X) { return search_smem_words(X, kStageWords) * 4; }
 
 __global__ void __launch_bounds__(kWarps * 32, 4)
-    search_y_kernel(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ near, uint32_t* __restrict__ field, int X,
-                    int Y, int Z, const uint32_t* __restrict__ skip) {
+    search_y_kernel(const uint32_t* bits, const uint32_t* near, uint32_t* field, int X, int Y, int Z, const uint32_t* skip) {
   extern __shared__ __align__(16) uint32_t s_rows[];
   if (skip != nullptr) {
     wait_for_previous();
-    if (*skip != 0u) return;
+    if (load_chained(skip) != 0u) return;
   }
   item_y(s_rows, bits, near, field, X, Y, Z, blockIdx.x, blockIdx.y);
 }
 
 __global__ void __launch_bounds__(kWarps * 32, 3)
-    search_x_kernel(const uint32_t* __restrict__ field, uint32_t* __restrict__ map, int X, int Y, int Z,
-                    const uint32_t* __restrict__ skip) {
+    search_x_kernel(const uint32_t* field, uint32_t* map, int X, int Y, int Z, const uint32_t* skip) {
   extern __shared__ __align__(16) uint32_t s_rows[];
   if (skip != nullptr) {
     wait_for_previous();
-    if (*skip != 0u) return;
+    if (load_chained(skip) != 0u) return;
   }
   item_x(s_rows, field, map, X, Y, Z, blockIdx.x, blockIdx.y);
 }
@@ -668,11 +676,10 @@ __global__ void zbits_insert_kernel(uint32_t* __restrict__ bits, int X, int Y, i
 // `near` from `bits`, one thread per (x, y) column (y fastest): one scan up
 // for the sites below each chunk, one down for those above.
 template <int kMaxChunks>
-__device__ __forceinline__ void near_column(const uint32_t* __restrict__ bits, uint32_t* __restrict__ near, uint32_t layer,
-                                            int chunks, uint32_t f) {
+__device__ __forceinline__ void near_column(const uint32_t* bits, uint32_t* near, uint32_t layer, int chunks, uint32_t f) {
   uint32_t m[kMaxChunks], below[kMaxChunks];
 #pragma unroll
-  for (int c = 0; c < kMaxChunks; ++c) m[c] = c < chunks ? __ldg(bits + (uint64_t)c * layer + f) : 0u;
+  for (int c = 0; c < kMaxChunks; ++c) m[c] = c < chunks ? load_chained(bits + (uint64_t)c * layer + f) : 0u;
   int last = -1;
 #pragma unroll
   for (int c = 0; c < kMaxChunks; ++c) {
@@ -688,10 +695,10 @@ __device__ __forceinline__ void near_column(const uint32_t* __restrict__ bits, u
 }
 
 template <int kMaxChunks>
-__global__ void __launch_bounds__(256) near_kernel(const uint32_t* __restrict__ bits, uint32_t* __restrict__ near,
-                                                   uint32_t layer, int chunks, const uint32_t* __restrict__ skip) {
+__global__ void __launch_bounds__(256) near_kernel(const uint32_t* bits, uint32_t* near, uint32_t layer, int chunks,
+                                                   const uint32_t* skip) {
   wait_for_previous();
-  if (skip != nullptr && *skip != 0u) return;
+  if (skip != nullptr && load_chained(skip) != 0u) return;
   const uint32_t f = blockIdx.x * blockDim.x + threadIdx.x;
   if (f < layer) near_column<kMaxChunks>(bits, near, layer, chunks, f);
 }
@@ -702,7 +709,7 @@ __global__ void __launch_bounds__(256) near_kernel(const uint32_t* __restrict__ 
 // flight) and stores the words with y fastest through shared memory.  With 32
 // y per block 320 x 320 x 96 made 300 blocks, two per SM (13.8 us, now 9.2).
 constexpr int kTileY = 8;
-__device__ __forceinline__ bool zbits_tile(const uint32_t* __restrict__ map, uint32_t* __restrict__ bits, int X, int Y, int Z,
+__device__ __forceinline__ bool zbits_tile(const uint32_t* __restrict__ vox, uint32_t* __restrict__ bits, int X, int Y, int Z,
                                            int bx, int by, int bz, uint32_t (&tile)[kTileY][33]) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int x = bx * 32 + lane, y = by * kTileY + warp, z0 = bz * 32;
@@ -710,11 +717,11 @@ __device__ __forceinline__ bool zbits_tile(const uint32_t* __restrict__ map, uin
   bool other = false;
   uint32_t word = 0u;
   if (x < X && y < Y) {
-    const uint32_t* src = map + (uint64_t)z0 * layer + (uint64_t)y * X + x;
+    vox += (uint64_t)z0 * layer + (uint64_t)y * X + x;
     const uint32_t own = (uint32_t)x | (uint32_t)y << 10 | (uint32_t)z0 << 20;
     uint32_t v[32];
 #pragma unroll
-    for (int i = 0; i < 32; ++i) v[i] = z0 + i < Z ? __ldg(src + (uint64_t)i * layer) : kDvUninit;
+    for (int i = 0; i < 32; ++i) v[i] = z0 + i < Z ? __ldg(vox + (uint64_t)i * layer) : kDvUninit;
 #pragma unroll
     for (int i = 0; i < 32; ++i) {
       if (v[i] != kDvUninit) {
@@ -809,7 +816,7 @@ __device__ __forceinline__ void near_map(const BatchMap& m) {
 __global__ void __launch_bounds__(256) near_batch_kernel(const BatchMap* __restrict__ maps, int skip_other) {
   const BatchMap m = maps[blockIdx.y];
   wait_for_previous();
-  if (skip_other && *other_flag(m) != 0u) return;
+  if (skip_other && load_chained(other_flag(m)) != 0u) return;
   const int chunks = z_chunks(m.Z);
   if (chunks <= 4) near_map<4>(m);
   else if (chunks <= 8) near_map<8>(m);
@@ -825,7 +832,7 @@ __global__ void __launch_bounds__(kWarps * 32, 4)
   const BatchMap m = maps[k];
   if (skip_other) {
     wait_for_previous();
-    if (*other_flag(m) != 0u) return;
+    if (load_chained(other_flag(m)) != 0u) return;
   }
   const int item = (int)((long long)blockIdx.x - __ldg(prefix + k)), c = item / m.X;
   const Areas a = areas(m);
@@ -840,7 +847,7 @@ __global__ void __launch_bounds__(kWarps * 32, 3)
   const BatchMap m = maps[k];
   if (skip_other) {
     wait_for_previous();
-    if (*other_flag(m) != 0u) return;
+    if (load_chained(other_flag(m)) != 0u) return;
   }
   const int item = (int)((long long)blockIdx.x - __ldg(prefix + k)), c = item / m.Y;
   item_x(s_rows, areas(m).field, m.vox, m.X, m.Y, m.Z, item - c * m.Y, c);
