@@ -694,27 +694,32 @@ bool list_by_bits(const gvx_blist* l, uint64_t total) {
 // before the list is written: 36 bytes each.
 constexpr uint64_t kUpperBoundEntries = 1ull << 20;
 
-gvx_status blist_insert_by_bits(gvx_blist* l, const float* d_xyz, uint64_t n, uint32_t meaning, cudaStream_t s) {
+// *done is left false, and the list as it was, where its ids turn out not to be
+// ascending voxels of the map (written through gvx_blist_data).
+gvx_status blist_insert_by_bits(gvx_blist* l, const float* d_xyz, uint64_t n, uint32_t meaning, cudaStream_t s, bool* done) {
   const uint64_t total = l->n + n;
   cudaError_t e = grow(&l->d_work, &l->work_bytes, list_bits_work_words(l->ref, l->n, n) * sizeof(uint32_t));
   if (e != cudaSuccess) return cuda_status(e, "list insert buffers");
   uint32_t* work = static_cast<uint32_t*>(l->d_work);
-  const uint32_t* d_total = nullptr;
-  uint32_t n_out = 0;
-  e = launch_list_mark(work, l->ref, l->side, d_xyz, n, l->d_ids, l->n, &d_total, s);
+  const uint32_t* d_result = nullptr;
+  struct {
+    uint32_t n_out, unusable;
+  } r = {0, 0};
+  e = launch_list_mark(work, l->ref, l->side, d_xyz, n, l->d_ids, l->n, &d_result, s);
   const uint64_t bound = std::min<uint64_t>(total, num_voxels(l->ref));
   if (e == cudaSuccess && bound <= kUpperBoundEntries) {
     e = blist_spare(l, bound);
   } else if (e == cudaSuccess) {
-    e = cudaMemcpyAsync(&n_out, d_total, sizeof(n_out), cudaMemcpyDeviceToHost, s);
+    e = cudaMemcpyAsync(&r, d_result, sizeof(r), cudaMemcpyDeviceToHost, s);
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // the merged list's length sizes its storage
-    if (e == cudaSuccess) e = blist_spare(l, n_out);
+    if (e == cudaSuccess) e = blist_spare(l, r.n_out);
   }
   if (e == cudaSuccess) e = launch_list_emit(work, l->ref, n, l->d_ids, l->d_vox, l->n, meaning, l->d_ids2, l->d_vox2, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(&n_out, d_total, sizeof(n_out), cudaMemcpyDeviceToHost, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(&r, d_result, sizeof(r), cudaMemcpyDeviceToHost, s);
   if (e == cudaSuccess) e = cudaStreamSynchronize(s);  // blocking, as the reference's insert
   if (e != cudaSuccess) return cuda_status(e, "list insert");
-  blist_adopt_spare(l, n_out);
+  *done = r.unusable == 0;
+  if (*done) blist_adopt_spare(l, r.n_out);
   return GVX_OK;
 }
 
@@ -730,7 +735,12 @@ gvx_status gvx_blist_insert_points(gvx_blist* l, const float* d_xyz, uint64_t n,
   cudaStream_t s = as_stream(stream);
   const uint64_t total = l->n + n;
   if (total >= 0xFFFFFFFFull) return fail(GVX_ERR_OUT_OF_DOMAIN, "list too long");
-  if (list_by_bits(l, total)) return blist_insert_by_bits(l, d_xyz, n, meaning, s);
+  if (list_by_bits(l, total)) {
+    bool done = false;
+    const gvx_status st = blist_insert_by_bits(l, d_xyz, n, meaning, s, &done);
+    if (st != GVX_OK || done) return st;
+    l->in_map = false;
+  }
   // work area: keys, vals, sorted keys, sorted vals, run heads, run positions
   // (total words each), then CUB's temporary storage
   size_t sort_bytes = 0, scan_bytes = 0;

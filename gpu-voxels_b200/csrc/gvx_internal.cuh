@@ -88,7 +88,7 @@ struct gvx_blist {
   uint32_t* d_ids2 = nullptr;
   uint8_t* d_vox2 = nullptr;
   uint64_t cap2 = 0;
-  bool in_map = true;  // every id is a voxel of the reference map (not known after gvx_blist_set)
+  bool in_map = true;  // ids as an insert leaves them: ascending voxels of the reference map (not after gvx_blist_set)
 };
 
 namespace gvx {
@@ -247,13 +247,14 @@ cudaError_t launch_list_list_types(const uint32_t* d_ids_a, const uint8_t* d_vox
 cudaError_t launch_extract_distances(const uint32_t* d_vox, gvx_dims d, int robot_radius, int8_t* d_out, cudaStream_t s);
 cudaError_t launch_init_floodfill(const int8_t* d_in, int16_t* d_out, uint64_t n, int robot_radius, cudaStream_t s);
 // List building by a bitmap of the reference map (list_bits.cu), for lists whose
-// ids are all voxels of it.  launch_list_mark merges the list's ids and the
-// points' into bits and leaves the merged length at *d_total (device);
+// ids are ascending voxels of it.  launch_list_mark merges the list's ids and the
+// points' into bits and leaves two words at *d_result (device): the merged length,
+// and whether the list's ids are something else (the merge is not to be used then);
 // launch_list_emit then writes the sorted unique ids and their voxels.
 // d_work: list_bits_work_words(...) words, 16-byte aligned.
 uint64_t list_bits_work_words(gvx_dims d, uint64_t n_old, uint64_t n);
 cudaError_t launch_list_mark(uint32_t* d_work, gvx_dims d, float side, const float* d_xyz, uint64_t n, const uint32_t* d_old,
-                             uint64_t n_old, const uint32_t** d_total, cudaStream_t s);
+                             uint64_t n_old, const uint32_t** d_result, cudaStream_t s);
 cudaError_t launch_list_emit(uint32_t* d_work, gvx_dims d, uint64_t n, const uint32_t* d_old, const uint8_t* d_old_vox,
                              uint64_t n_old, uint32_t meaning, uint32_t* d_ids, uint8_t* d_vox, cudaStream_t s);
 // Distance band -> list: per-tile counts, exclusive tile offsets (+ total at

@@ -8,6 +8,11 @@
 // voxel is the list's old voxel, found back by the rank of its bit, with the new
 // meaning set where a point fell.
 //
+// That holds for ascending ids inside the map.  The ids lie in storage that a
+// caller may write (gvx_blist_data), so the mark kernel checks them, uses none
+// that fails, and reports it beside the merged length: the sort takes the list
+// then.
+//
 // What bounds it: launches (seven short ones and one wait) while the map has
 // few million voxels; then the bitmap, read twice after it is cleared.  The sort
 // of (id, index) pairs it replaces (radix sort, run heads, scan, merge, two
@@ -27,15 +32,21 @@ constexpr int kTileWords = 1024;  // bitmap words per block of 256 threads
 constexpr uint32_t kOutside = 0xffffffffu;
 
 // Old ids and points to bits; keys[i] = point i's id, kOutside out of bounds
-// (remove_out_of_bounds, TemplateVoxelList.hpp:318-341).
+// (remove_out_of_bounds, TemplateVoxelList.hpp:318-341).  *unusable is set
+// where an old id is no voxel of the map or not above the one before it.
 __global__ void list_mark_kernel(const float* __restrict__ xyz, uint64_t n, gvx_dims d, float side,
                                  const uint32_t* __restrict__ old_ids, uint64_t n_old, uint32_t* __restrict__ keys,
-                                 uint32_t* __restrict__ bits) {
+                                 uint32_t* __restrict__ bits, uint32_t* __restrict__ unusable) {
   const uint64_t total = n_old + n;
+  const uint32_t n_vox = d.x * d.y * d.z;  // below 2^30
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < total; i += (uint64_t)gridDim.x * blockDim.x) {
     uint32_t id;
     if (i < n_old) {
       id = old_ids[i];
+      if (id >= n_vox || (i > 0 && old_ids[i - 1] >= id)) {
+        *unusable = 1u;
+        id = kOutside;
+      }
     } else {
       const uint64_t p = i - n_old;
       const uint32_t x = coord_to_voxel(xyz[3 * p], side), y = coord_to_voxel(xyz[3 * p + 1], side),
@@ -87,8 +98,10 @@ __global__ void __launch_bounds__(256) bits_count_kernel(const uint32_t* __restr
   if (threadIdx.x == 0) tiles[blockIdx.x] = sum;
 }
 
-// Exclusive scan of the tile counts by one block; the total goes to tiles[n].
-__global__ void __launch_bounds__(1024) tiles_scan_kernel(uint32_t* __restrict__ tiles, uint32_t n) {
+// Exclusive scan of the tile counts by one block; the total goes to tiles[n]
+// and beside it, for one read-back, the mark kernel's flag.
+__global__ void __launch_bounds__(1024) tiles_scan_kernel(uint32_t* __restrict__ tiles, uint32_t n,
+                                                          const uint32_t* __restrict__ unusable) {
   __shared__ uint32_t warp_sum[32];
   __shared__ uint32_t carry;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -111,7 +124,10 @@ __global__ void __launch_bounds__(1024) tiles_scan_kernel(uint32_t* __restrict__
     if (threadIdx.x == 1023) carry = before + inc;
   }
   __syncthreads();
-  if (threadIdx.x == 0) tiles[n] = carry;
+  if (threadIdx.x == 0) {
+    tiles[n] = carry;
+    tiles[n + 1] = *unusable;
+  }
 }
 
 // Ids of the tile's bits in order and `fill` for each of their voxels; ranks
@@ -138,10 +154,11 @@ __device__ __forceinline__ uint64_t rank_of(const uint32_t* __restrict__ bits, c
   return (uint64_t)ranks[id >> 5] + __popc(bits[id >> 5] & ((1u << (id & 31)) - 1u));
 }
 
-// The old entries' voxels at their new places.
+// The old entries' voxels at their new places (an unusable id has none).
 __global__ void list_move_kernel(const uint32_t* __restrict__ bits, const uint32_t* __restrict__ ranks,
                                  const uint32_t* __restrict__ old_ids, const uint4* __restrict__ old_vox, uint64_t n_old,
-                                 uint4* __restrict__ vox) {
+                                 uint4* __restrict__ vox, const uint32_t* __restrict__ unusable) {
+  if (*unusable != 0u) return;
   for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n_old; i += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t k = rank_of(bits, ranks, old_ids[i]);
     vox[2 * k] = old_vox[2 * i];
@@ -167,42 +184,51 @@ uint64_t align64(uint64_t words) { return (words + 63) / 64 * 64; }
 uint64_t bitmap_words(gvx_dims d) { return (num_voxels(d) + 31) / 32; }
 uint64_t bitmap_tiles(gvx_dims d) { return (bitmap_words(d) + kTileWords - 1) / kTileWords; }
 
+// The work area: bits and behind them the flag, tile counts with the merged
+// length and the flag again, the points' ids, and (for a list with entries) ranks.
+struct Layout {
+  uint64_t tiles, keys, ranks, words;
+  Layout(gvx_dims d, uint64_t n_old, uint64_t n)
+      : tiles(align64(bitmap_words(d) + 1)),
+        keys(tiles + align64(bitmap_tiles(d) + 2)),
+        ranks(keys + align64(n)),
+        words(ranks + (n_old ? bitmap_words(d) : 0)) {}
+};
+
 }  // namespace
 
-uint64_t list_bits_work_words(gvx_dims d, uint64_t n_old, uint64_t n) {
-  return align64(bitmap_words(d)) + align64(bitmap_tiles(d) + 1) + align64(n) + (n_old ? bitmap_words(d) : 0);
-}
+uint64_t list_bits_work_words(gvx_dims d, uint64_t n_old, uint64_t n) { return Layout(d, n_old, n).words; }
 
 cudaError_t launch_list_mark(uint32_t* d_work, gvx_dims d, float side, const float* d_xyz, uint64_t n, const uint32_t* d_old,
-                             uint64_t n_old, const uint32_t** d_total, cudaStream_t s) {
-  uint32_t* bits = d_work;
-  uint32_t* tiles = bits + align64(bitmap_words(d));
-  uint32_t* keys = tiles + align64(bitmap_tiles(d) + 1);
+                             uint64_t n_old, const uint32_t** d_result, cudaStream_t s) {
+  const Layout w(d, n_old, n);
+  uint32_t *bits = d_work, *unusable = bits + bitmap_words(d), *tiles = d_work + w.tiles;
   const uint32_t nt = (uint32_t)bitmap_tiles(d);
-  *d_total = tiles + nt;
-  const cudaError_t e = cudaMemsetAsync(bits, 0, bitmap_words(d) * sizeof(uint32_t), s);
+  *d_result = tiles + nt;
+  const cudaError_t e = cudaMemsetAsync(bits, 0, (bitmap_words(d) + 1) * sizeof(uint32_t), s);
   if (e != cudaSuccess) return e;
-  list_mark_kernel<<<grid_for(n_old + n), 256, 0, s>>>(d_xyz, n, d, side, d_old, n_old, keys, bits);
+  list_mark_kernel<<<grid_for(n_old + n), 256, 0, s>>>(d_xyz, n, d, side, d_old, n_old, d_work + w.keys, bits, unusable);
   bits_count_kernel<<<nt, 256, 0, s>>>(bits, bitmap_words(d), tiles);
-  tiles_scan_kernel<<<1, 1024, 0, s>>>(tiles, nt);
+  tiles_scan_kernel<<<1, 1024, 0, s>>>(tiles, nt, unusable);
   return cudaGetLastError();
 }
 
 cudaError_t launch_list_emit(uint32_t* d_work, gvx_dims d, uint64_t n, const uint32_t* d_old, const uint8_t* d_old_vox,
                              uint64_t n_old, uint32_t meaning, uint32_t* d_ids, uint8_t* d_vox, cudaStream_t s) {
-  const uint32_t* bits = d_work;
-  const uint32_t* tiles = bits + align64(bitmap_words(d));
-  const uint32_t* keys = tiles + align64(bitmap_tiles(d) + 1);
-  uint32_t* ranks = n_old ? d_work + align64(bitmap_words(d)) + align64(bitmap_tiles(d) + 1) + align64(n) : nullptr;
+  const Layout w(d, n_old, n);
+  const uint32_t *bits = d_work, *unusable = bits + bitmap_words(d);
+  uint32_t* ranks = n_old ? d_work + w.ranks : nullptr;
   uint32_t f[kBitVoxelWords] = {};
   if (n_old == 0) f[meaning >> 5] = 1u << (meaning & 31);  // every entry holds a new point
-  bits_emit_kernel<<<(unsigned)bitmap_tiles(d), 256, 0, s>>>(bits, bitmap_words(d), tiles, make_uint4(f[0], f[1], f[2], f[3]),
+  bits_emit_kernel<<<(unsigned)bitmap_tiles(d), 256, 0, s>>>(bits, bitmap_words(d), d_work + w.tiles,
+                                                             make_uint4(f[0], f[1], f[2], f[3]),
                                                              make_uint4(f[4], f[5], f[6], f[7]), d_ids,
                                                              reinterpret_cast<uint4*>(d_vox), ranks);
   if (n_old) {
     list_move_kernel<<<grid_for(n_old), 256, 0, s>>>(bits, ranks, d_old, reinterpret_cast<const uint4*>(d_old_vox), n_old,
-                                                     reinterpret_cast<uint4*>(d_vox));
-    list_meaning_kernel<<<grid_for(n), 256, 0, s>>>(bits, ranks, keys, n, meaning, reinterpret_cast<uint32_t*>(d_vox));
+                                                     reinterpret_cast<uint4*>(d_vox), unusable);
+    list_meaning_kernel<<<grid_for(n), 256, 0, s>>>(bits, ranks, d_work + w.keys, n, meaning,
+                                                    reinterpret_cast<uint32_t*>(d_vox));
   }
   return cudaGetLastError();
 }

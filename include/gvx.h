@@ -424,6 +424,10 @@ GVX_API gvx_status gvx_blist_create(const gvx_dims *ref_dims, float voxel_side, 
 GVX_API gvx_status gvx_blist_destroy(gvx_blist *l);
 /* Number of (unique) entries; synchronises the list's last update. */
 GVX_API gvx_status gvx_blist_size(const gvx_blist *l, uint64_t *n);
+/* The entries' ids (ascending, unique) and voxels, valid until the next call
+ * that changes the list's length.  Both may be written in place; ids left
+ * unsorted, repeated or outside the reference map are sorted and merged by the
+ * next insert. */
 GVX_API gvx_status gvx_blist_data(const gvx_blist *l, uint32_t **d_ids, uint8_t **d_voxels);
 GVX_API gvx_status gvx_blist_clear(gvx_blist *l);
 /* Replaces TemplateVoxelList::insertPointCloud (GV/voxellist/TemplateVoxelList.hpp:363-393):
