@@ -333,12 +333,15 @@ int configs_per_block(uint64_t n) {
   return kWarpsPerBlock * (int)std::min<uint64_t>(each, kMaxBlockConfigs / kWarpsPerBlock);
 }
 
-// The dynamic shared memory limit, raised once per kernel and device where an
-// arm needs more than the 48 KB every kernel may use.
+// The dynamic shared memory limit of a kernel, for arms that need more than the
+// 48 KB every kernel may use.  The limit is the kernel's, not the call's, so every
+// call raises it to the largest arm's size: with its own size a call would lower
+// it between another thread's call here and that thread's launch.
 template <auto kKernel>
 cudaError_t allow_smem(size_t bytes) {
+  constexpr auto kLimit = cudaFuncAttributeMaxDynamicSharedMemorySize;
   return bytes <= 48 * 1024 ? cudaSuccess
-                            : cudaFuncSetAttribute(kKernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
+                            : cudaFuncSetAttribute(kKernel, kLimit, (int)arm_smem_bytes(GVX_MAX_JOINTS, GVX_MAX_SPHERES, kMaxBlockConfigs));
 }
 
 template <int kJ>
