@@ -246,13 +246,15 @@ gvx_status gvx_batch_autotune(gvx_batch* b, int force, gvx_edt_config* out, gvx_
       return r;
     };
     if (e == cudaSuccess) e = copy_all(true);
+    BatchItems sweeps = b->items;  // timed also where the row search takes the maps, as for one map
+    sweeps.search = false;
     best_ms = 1e30f;
     for (int rows : {16, 32}) {
       float t_min = 1e30f;
       for (int rep = 0; rep < 4 && e == cudaSuccess; ++rep) {  // first run warms up
         e = copy_all(false);
         if (e == cudaSuccess) e = cudaEventRecord(e0, s);
-        if (e == cudaSuccess) e = launch_edt_batch(b->d_table, b->items, s, rows);
+        if (e == cudaSuccess) e = launch_edt_batch(b->d_table, sweeps, s, rows);
         if (e == cudaSuccess) e = cudaEventRecord(e1, s);
         if (e == cudaSuccess) e = cudaEventSynchronize(e1);
         float ms = 0.f;

@@ -1587,13 +1587,17 @@ cudaError_t launch_edt_pass(uint32_t* d_vox, uint32_t* d_scratch, uint64_t scrat
   return launch_sweep_pass(d_vox, d_scratch, scratch_words, d, pass, s, rows, nullptr);
 }
 
+cudaError_t launch_edt_sweeps(uint32_t* d_vox, uint32_t* d_scratch, uint64_t scratch_words, gvx_dims d, cudaStream_t s,
+                              const EdtConfig& cfg) {
+  if (scratch_words < edt_scratch_words_min(d)) return cudaErrorInvalidValue;
+  const cudaError_t e = launch_pass_z(d_vox, d_scratch, d, s);
+  return e == cudaSuccess ? launch_sweeps(d_vox, d_scratch, scratch_words, d, s, cfg, nullptr) : e;
+}
+
 cudaError_t launch_edt(uint32_t* d_vox, uint32_t* d_scratch, uint64_t scratch_words, gvx_dims d, cudaStream_t s,
                        const EdtConfig& cfg) {
   if (scratch_words < edt_scratch_words_min(d)) return cudaErrorInvalidValue;
-  if (!use_search(d, scratch_words)) {
-    const cudaError_t e = launch_pass_z(d_vox, d_scratch, d, s);
-    return e == cudaSuccess ? launch_sweeps(d_vox, d_scratch, scratch_words, d, s, cfg, nullptr) : e;
-  }
+  if (!use_search(d, scratch_words)) return launch_edt_sweeps(d_vox, d_scratch, scratch_words, d, s, cfg);
   // The row search takes a map whose sites are all their own voxels; the flag
   // it sets otherwise lets the general pass Z and the sweeps run.
   uint32_t* other = d_scratch + (uint64_t)d.z + 2;

@@ -157,6 +157,9 @@ struct EdtConfig {
 };
 cudaError_t launch_edt(uint32_t* d_vox, uint32_t* d_scratch, uint64_t scratch_words, gvx_dims d, cudaStream_t s,
                        const EdtConfig& cfg = EdtConfig{});
+// The same by the sweeps whatever the map holds (what an EdtConfig is timed on).
+cudaError_t launch_edt_sweeps(uint32_t* d_vox, uint32_t* d_scratch, uint64_t scratch_words, gvx_dims d, cudaStream_t s,
+                              const EdtConfig& cfg);
 // pass 0 = Z (occupancy bits from the map, the bits pass, and the general
 // pass when a voxel holds another site), 1 = Y, 2 = X, 3 = fused Y -> X
 cudaError_t launch_edt_pass(uint32_t* d_vox, uint32_t* d_scratch, uint64_t scratch_words, gvx_dims d, int pass,

@@ -1,6 +1,8 @@
 // EDT autotuner: picks the sweep configuration (rows per staging chunk, fused
-// or separate y/x launches) by timing every candidate on a copy of the map's
-// current content.  Results are bit-identical for every candidate; only the
+// or separate y/x launches) by timing the sweeps with every candidate on a copy
+// of the map's current content -- the sweeps also where the row search would
+// take that content: the choice is for the maps of these dims that hold other
+// sites, and the search has no setting to time.  Results are bit-identical for every candidate; only the
 // speed differs.  Choices are cached per (device, dims) in memory and, when
 // the environment variable GVX_TUNE_CACHE names a file, in that file (one
 // line per entry: key rows fused ms), so later processes skip the timing.
@@ -204,7 +206,7 @@ gvx_status gvx_dvm_autotune(gvx_dvm* m, int force, gvx_edt_config* out, gvx_stre
       for (int rep = 0; rep < 4 && e == cudaSuccess; ++rep) {  // first run warms up
         e = cudaMemcpyAsync(tmp, m->d_vox, n * sizeof(uint32_t), cudaMemcpyDeviceToDevice, s);
         if (e == cudaSuccess) e = cudaEventRecord(e0, s);
-        if (e == cudaSuccess) e = launch_edt(tmp, m->d_scratch, m->scratch_words, m->dims, s, cands[c]);
+        if (e == cudaSuccess) e = launch_edt_sweeps(tmp, m->d_scratch, m->scratch_words, m->dims, s, cands[c]);
         if (e == cudaSuccess) e = cudaEventRecord(e1, s);
         if (e == cudaSuccess) e = cudaEventSynchronize(e1);
         float ms = 0.f;

@@ -117,8 +117,8 @@ typedef struct {
   float ms;
 } gvx_edt_config;
 /* Project-written autotuner (no counterpart in the reference, whose PBA band
- * counts are fixed by the caller): times every configuration on a copy of
- * the map's current content (allocated for the call and freed; the map is
+ * counts are fixed by the caller): times the sweeps at every configuration on
+ * a copy of the map's current content (allocated for the call and freed; the map is
  * not modified), keeps the fastest for this map's later EDTs and returns it.
  * Choices are cached per device and dims in memory and, if the environment
  * variable GVX_TUNE_CACHE names a file, across processes; force = 1 re-times.

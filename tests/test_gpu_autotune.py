@@ -99,6 +99,61 @@ def test_batch_autotune_restores_maps_and_stays_exact():
         assert np.array_equal(to_u32(maps[k].data()), want), dims
 
 
+def _ms(fn, before=lambda: None):
+    best = 1e9
+    for _ in range(6):
+        before()
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        a.record()
+        fn()
+        b.record()
+        torch.cuda.synchronize()
+        best = min(best, a.elapsed_time(b))
+    return best
+
+
+def test_tuner_times_the_sweeps_of_a_map_the_row_search_takes():
+    """The configuration is the sweeps'.  Timing the EDT of an inserted map, which the row search takes, would time
+    the same kernels four times (a fourth of the sweeps' time at these dims) and choose by noise."""
+    dims = (128, 128, 128)
+    pts = torch.as_tensor(_scene(dims, 3, 50_000)).cuda()
+    m = gvx.DistanceVoxelMap(dims, 0.01)
+    m.insertPointCloud(pts)
+    cfg = m.autotune(force=True)
+
+    def fill():
+        m.clearMap()
+        m.insertPointCloud(pts)
+
+    def sweeps():
+        m.edt_pass(0)
+        for p in ((3,) if cfg["fused"] else (1, 2)):
+            m.edt_pass(p)
+
+    swept, searched = _ms(sweeps, fill), _ms(m.parallelBanding3D, fill)
+    assert searched < 0.5 * swept
+    assert 0.7 * swept < cfg["ms"] < 1.4 * swept
+    assert m.edt_check() == 0
+
+
+def test_batch_tuner_times_the_sweeps():
+    dims = [(128, 120, 100), (96, 128, 64), (100, 90, 128)]
+    clouds = [_scene(d, 5 + i, 20_000) for i, d in enumerate(dims)]
+    maps = [gvx.DistanceVoxelMap(d, 0.01) for d in dims]
+    b = Batch(maps)
+    pts = torch.as_tensor(np.concatenate(clouds)).cuda()
+    offs = torch.as_tensor(np.concatenate([[0], np.cumsum([len(c) for c in clouds])]).astype(np.int64)).cuda()
+
+    def fill():
+        b.clear()
+        b.insert(pts, offs)
+
+    fill()
+    cfg = b.autotune(force=True)
+    assert cfg["ms"] > 1.5 * _ms(b.edt, fill)
+    assert b.edt_check() == 0
+
+
 def test_query_launch_shapes_are_bit_identical_and_autotune_picks_one():
     dims = (90, 70, 50)
     pts = _scene(dims, 7)
