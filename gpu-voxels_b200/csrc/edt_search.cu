@@ -769,12 +769,17 @@ __device__ __forceinline__ uint32_t owner(const T* __restrict__ prefix, uint32_t
   return lo;
 }
 
-__global__ void zbits_clear_batch_kernel(const BatchMap* __restrict__ maps) {
-  const BatchMap m = maps[blockIdx.y];
-  if (blockIdx.x == 0 && threadIdx.x == 0) *other_flag(m) = 0u;
-  uint32_t* bits = areas(m).bits;
-  const uint64_t n = bits_words(m.X, m.Y, m.Z);
-  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) bits[i] = 0u;
+// Block rows of the kernels below: row r takes the maps r, r + gridDim.y, ..
+unsigned map_rows(uint32_t n_maps) { return std::min(n_maps, 65535u); }
+
+__global__ void zbits_clear_batch_kernel(const BatchMap* __restrict__ maps, uint32_t n_maps) {
+  for (uint32_t k = blockIdx.y; k < n_maps; k += gridDim.y) {
+    const BatchMap m = maps[k];
+    if (blockIdx.x == 0 && threadIdx.x == 0) *other_flag(m) = 0u;
+    uint32_t* bits = areas(m).bits;
+    const uint64_t n = bits_words(m.X, m.Y, m.Z);
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) bits[i] = 0u;
+  }
 }
 
 // point i belongs to map k with offsets[k] <= i < offsets[k + 1]
@@ -790,18 +795,20 @@ __global__ void zbits_insert_batch_kernel(const BatchMap* __restrict__ maps, uin
   }
 }
 
-// block row = map; the blocks of a row stride over the map's tiles
-__global__ void __launch_bounds__(256) zbits_from_map_batch_kernel(const BatchMap* __restrict__ maps) {
+// the blocks of a row stride over its map's tiles
+__global__ void __launch_bounds__(256) zbits_from_map_batch_kernel(const BatchMap* __restrict__ maps, uint32_t n_maps) {
   __shared__ uint32_t tile[kTileY][33];
-  const BatchMap m = maps[blockIdx.y];
-  uint32_t* bits = areas(m).bits;
-  const int tx = (m.X + 31) >> 5, ty = (m.Y + kTileY - 1) / kTileY, tiles = tx * ty * z_chunks(m.Z);
-  bool other = false;
-  for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
-    other |= zbits_tile(m.vox, bits, m.X, m.Y, m.Z, t % tx, t / tx % ty, t / (tx * ty), tile);
-    __syncthreads();
+  for (uint32_t k = blockIdx.y; k < n_maps; k += gridDim.y) {
+    const BatchMap m = maps[k];
+    uint32_t* bits = areas(m).bits;
+    const int tx = (m.X + 31) >> 5, ty = (m.Y + kTileY - 1) / kTileY, tiles = tx * ty * z_chunks(m.Z);
+    bool other = false;
+    for (int t = blockIdx.x; t < tiles; t += gridDim.x) {
+      other |= zbits_tile(m.vox, bits, m.X, m.Y, m.Z, t % tx, t / tx % ty, t / (tx * ty), tile);
+      __syncthreads();
+    }
+    if (__any_sync(kFullMask, other) && (threadIdx.x & 31) == 0) atomicOr(other_flag(m), 1u);
   }
-  if (__any_sync(kFullMask, other) && (threadIdx.x & 31) == 0) atomicOr(other_flag(m), 1u);
 }
 
 template <int kMaxChunks>
@@ -812,16 +819,18 @@ __device__ __forceinline__ void near_map(const BatchMap& m) {
     near_column<kMaxChunks>(a.bits, a.near, layer, z_chunks(m.Z), f);
 }
 
-// block row = map, each with the registers and loads of its own height
-__global__ void __launch_bounds__(256) near_batch_kernel(const BatchMap* __restrict__ maps, int skip_other) {
-  const BatchMap m = maps[blockIdx.y];
+// each map with the registers and loads of its own height
+__global__ void __launch_bounds__(256) near_batch_kernel(const BatchMap* __restrict__ maps, uint32_t n_maps, int skip_other) {
   wait_for_previous();
-  if (skip_other && load_chained(other_flag(m)) != 0u) return;
-  const int chunks = z_chunks(m.Z);
-  if (chunks <= 4) near_map<4>(m);
-  else if (chunks <= 8) near_map<8>(m);
-  else if (chunks <= 16) near_map<16>(m);
-  else near_map<32>(m);
+  for (uint32_t k = blockIdx.y; k < n_maps; k += gridDim.y) {
+    const BatchMap m = maps[k];
+    if (skip_other && load_chained(other_flag(m)) != 0u) continue;
+    const int chunks = z_chunks(m.Z);
+    if (chunks <= 4) near_map<4>(m);
+    else if (chunks <= 8) near_map<8>(m);
+    else if (chunks <= 16) near_map<16>(m);
+    else near_map<32>(m);
+  }
 }
 
 __global__ void __launch_bounds__(kWarps * 32, 4)
@@ -948,7 +957,7 @@ namespace {
 cudaError_t launch_from_bits_batch(const BatchMap* d_table, const BatchItems& it, int skip_other, cudaStream_t s) {
   cudaError_t e = search_setup_once();
   if (e != cudaSuccess) return e;
-  e = launch_next(near_batch_kernel, dim3(128, it.n_maps), 0, s, d_table, skip_other);
+  e = launch_next(near_batch_kernel, dim3(128, map_rows(it.n_maps)), 0, s, d_table, it.n_maps, skip_other);
   if (e == cudaSuccess)
     e = launch_next(search_y_batch_kernel, dim3((unsigned)it.total[4]), smem_y((int)it.y_max), s, d_table, it.d_prefix[4],
                     it.n_maps, skip_other);
@@ -961,7 +970,7 @@ cudaError_t launch_from_bits_batch(const BatchMap* d_table, const BatchItems& it
 
 cudaError_t launch_search_voxelize_batch(const BatchMap* d_table, const BatchItems& it, const float* d_xyz,
                                          const uint64_t* d_offsets, uint64_t n_total, cudaStream_t s) {
-  zbits_clear_batch_kernel<<<dim3(64, it.n_maps), 256, 0, s>>>(d_table);
+  zbits_clear_batch_kernel<<<dim3(64, map_rows(it.n_maps)), 256, 0, s>>>(d_table, it.n_maps);
   if (n_total > 0) {
     const unsigned blocks = (unsigned)std::min<uint64_t>((n_total + 255) / 256, (uint64_t)device_sms() * 16);
     zbits_insert_batch_kernel<<<blocks, 256, 0, s>>>(d_table, it.n_maps, d_xyz, d_offsets, n_total);
@@ -971,7 +980,7 @@ cudaError_t launch_search_voxelize_batch(const BatchMap* d_table, const BatchIte
 }
 
 cudaError_t launch_search_filled_batch(const BatchMap* d_table, const BatchItems& it, cudaStream_t s) {
-  zbits_from_map_batch_kernel<<<dim3(64, it.n_maps), 256, 0, s>>>(d_table);
+  zbits_from_map_batch_kernel<<<dim3(64, map_rows(it.n_maps)), 256, 0, s>>>(d_table, it.n_maps);
   const cudaError_t e = cudaGetLastError();
   return e == cudaSuccess ? launch_from_bits_batch(d_table, it, 1, s) : e;
 }

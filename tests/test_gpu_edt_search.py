@@ -94,3 +94,18 @@ def test_batch_search_equals_oracle(long_map):
     for m, d, w in zip(maps, dims, wants):
         assert np.array_equal(to_u32(m.data()), w), first_mismatch(to_u32(m.data()), w, d)
     assert b.edt_check() == 0
+
+
+@pytest.mark.gpu
+def test_batch_of_more_maps_than_block_rows():
+    """A launch has at most 65,535 block rows; a batch has no such limit."""
+    n = 65_540
+    rng = np.random.default_rng(1)
+    voxels = torch.full((n, 8), 0x3FFFFFFF, dtype=torch.int32, device="cuda")  # 5 x 1 x 1 maps, 32 bytes apart
+    site = torch.as_tensor(rng.integers(0, 5, n)).cuda()
+    voxels.scatter_(1, site[:, None], site[:, None].to(torch.int32))
+    maps = [gvx.DistanceVoxelMap((5, 1, 1), 1.0, voxels=voxels[k, :5]) for k in range(n)]
+    b = Batch(maps)
+    b.edt()
+    assert b.edt_check() == 0
+    assert torch.equal(voxels[:, :5].long(), site[:, None].expand(n, 5))
