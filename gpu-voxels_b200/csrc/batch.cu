@@ -77,6 +77,32 @@ __global__ void batch_trilinear_kernel(const BatchMap* __restrict__ maps, const 
 
 int sms() { return device_sms(); }
 
+// Whether the row search or the sweeps take a batch whose maps both can take.  A
+// search block costs much the same however few of its 32 z and of its rows a map
+// fills, and a sweep's warp packs the columns of several slices; but a sweep walks
+// its rows one after another however few warps there are.  So many small or flat
+// maps are the sweeps', few maps and larger ones the search's.  The costs (ns of a
+// filled B200 per block of a pass and per warp of a sweep, and per row that a lone
+// warp walks) were fitted to batches of one kind at about 1 % occupancy.
+// Search against sweeps, us: 2000 of 12^3 478 : 229, 300 of 20^3 125 : 104, 64 of
+// 100 x 100 x 8 196 : 191, 300 of 32^3 198 : 230, 100 of 48^3 200 : 238, 100 of
+// 64^3 295 : 455, 64 of 96^3 566 : 824, 16 of 64^3 58 : 134, 4 of 30 x 25 x 20 19 : 55.
+// Nearly empty maps (10 points each) gain less: 100 of 64^3 287 : 210.
+bool search_is_faster(gvx_dvm* const* maps, uint32_t n_maps) {
+  auto block_ns = [](uint32_t rows) { return 8.5 + 0.125 * std::max(0, (int)rows - 48); };
+  auto warp_ns = [](uint32_t rows) { return 6.0 + 0.16 * rows; };
+  double search = 0.0, sweeps = 0.0;
+  uint32_t x_max = 1, y_max = 1;
+  for (uint32_t k = 0; k < n_maps; ++k) {
+    const gvx_dims& d = maps[k]->dims;
+    search += search_items(d, 1) * block_ns(d.y) + search_items(d, 2) * block_ns(d.x);
+    sweeps += edt_pass_items(d, 1) * warp_ns(d.y) + edt_pass_items(d, 2) * warp_ns(d.x);
+    x_max = std::max(x_max, d.x);
+    y_max = std::max(y_max, d.y);
+  }
+  return search < std::max(sweeps, 600.0 * (x_max + y_max));
+}
+
 gvx_status fail(gvx_status st, const char* msg) {
   set_error(msg);
   return st;
@@ -160,7 +186,7 @@ gvx_status gvx_batch_create(gvx_dvm* const* maps, uint32_t n_maps, gvx_batch** o
   b->items.x_max = x_max;
   b->items.y_max = y_max;
   b->items.z_max = z_max;
-  b->items.search = search && b->items.total[4] < (1ll << 31) && b->items.total[5] < (1ll << 31);
+  b->items.search = search && search_is_faster(maps, n_maps) && b->items.total[4] < (1ll << 31) && b->items.total[5] < (1ll << 31);
   *out = b;
   return GVX_OK;
 }

@@ -99,13 +99,63 @@ def test_batch_search_equals_oracle(long_map):
 @pytest.mark.gpu
 def test_batch_of_more_maps_than_block_rows():
     """A launch has at most 65,535 block rows; a batch has no such limit."""
-    n = 65_540
-    rng = np.random.default_rng(1)
-    voxels = torch.full((n, 8), 0x3FFFFFFF, dtype=torch.int32, device="cuda")  # 5 x 1 x 1 maps, 32 bytes apart
-    site = torch.as_tensor(rng.integers(0, 5, n)).cuda()
-    voxels.scatter_(1, site[:, None], site[:, None].to(torch.int32))
-    maps = [gvx.DistanceVoxelMap((5, 1, 1), 1.0, voxels=voxels[k, :5]) for k in range(n)]
+    n, dims = 65_540, (18, 18, 32)  # dims at which the row search takes the batch
+    n_vox = dims[0] * dims[1] * dims[2]
+    voxels = torch.full((n, n_vox), 0x3FFFFFFF, dtype=torch.int32, device="cuda")
+    at = torch.as_tensor(np.random.default_rng(1).integers(0, n_vox, n)).cuda()
+    site = (at % dims[0] | at // dims[0] % dims[1] << 10 | at // (dims[0] * dims[1]) << 20).to(torch.int32)[:, None]
+    voxels.scatter_(1, at[:, None], site)
+    maps = [gvx.DistanceVoxelMap(dims, 1.0, voxels=voxels[k]) for k in range(n)]
     b = Batch(maps)
     b.edt()
     assert b.edt_check() == 0
-    assert torch.equal(voxels[:, :5].long(), site[:, None].expand(n, 5))
+    assert all(bool((v == s).all()) for v, s in zip(voxels.split(4096), site.split(4096)))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims,n", [((12, 12, 12), 500), ((20, 20, 20), 100), ((64, 50, 4), 30), ((5, 3, 1), 300)])
+def test_batches_of_small_maps_equal_oracle(dims, n):
+    """Many small or flat maps, which the sweeps take, a third of them transformed before."""
+    clouds = [_points(dims, 1 + i % 40, i) for i in range(n)]
+    maps = [gvx.DistanceVoxelMap(dims, SIDE) for _ in range(n)]
+    b = Batch(maps)
+    xyz = torch.as_tensor(np.concatenate(clouds)).cuda()
+    offsets = torch.tensor(np.concatenate([[0], np.cumsum([len(c) for c in clouds])]), dtype=torch.int64).cuda()
+    wants = [oracle_edt(dims, SIDE, c)[1] for c in clouds]
+    b.voxelize_edt(xyz, offsets)
+    assert np.array_equal(np.stack([to_u32(m.data()) for m in maps]), np.stack(wants))
+    b.clear()
+    b.insert(xyz, offsets)
+    for m, w in list(zip(maps, wants))[::3]:
+        m.parallelBanding3D()
+        oracle.pba(w, dims)
+    b.edt()
+    assert np.array_equal(np.stack([to_u32(m.data()) for m in maps]), np.stack(wants))
+    assert b.edt_check() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims,n", [((12, 12, 12), 2000), ((20, 20, 20), 300), ((100, 100, 8), 64), ((48, 48, 48), 100),
+                                    ((96, 96, 96), 32), ((128, 128, 128), 2)])
+def test_batches_take_the_faster_way(dims, n):
+    """Whatever the maps' sizes, the batched EDT takes no longer than the sweeps (which the tuner times) by more than a
+    fourth, a few launches' time apart.  Taken by the row search, 2000 maps of 12^3 took three times as long."""
+    clouds = [_points(dims, max(10, dims[0] * dims[1] * dims[2] // 100), i) for i in range(n)]
+    maps = [gvx.DistanceVoxelMap(dims, SIDE) for _ in range(n)]
+    b = Batch(maps)
+    xyz = torch.as_tensor(np.concatenate(clouds)).cuda()
+    offsets = torch.tensor(np.concatenate([[0], np.cumsum([len(c) for c in clouds])]), dtype=torch.int64).cuda()
+    b.clear()
+    b.insert(xyz, offsets)
+    sweeps = b.autotune(force=True)["ms"]
+    best = 1e9
+    for _ in range(6):
+        b.clear()
+        b.insert(xyz, offsets)
+        t0, t1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        t0.record()
+        b.edt()
+        t1.record()
+        torch.cuda.synchronize()
+        best = min(best, t0.elapsed_time(t1))
+    assert best < 1.25 * sweeps + 0.02
