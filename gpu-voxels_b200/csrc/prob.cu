@@ -36,7 +36,10 @@ __device__ __forceinline__ int prob_steps(int cur, int mode, int delta, int time
 // one compare-and-swap by the first of them: points of a sensor frame that
 // follow each other mostly fall in one voxel, and a lane of its own for each
 // made them retry against each other, an L2 round trip per try (307k points of
-// four depth images: 23.4 us, now 8.6).
+// four depth images: 23.4 us, now 8.6).  Where no lane's update changes its voxel
+// (the updates of a call go one way, so a saturated voxel stays so) the warp has
+// nothing to group: a map that has settled is only read (3M random points into a
+// settled 256^3 map 20 us, 38 with the grouping; a fresh one 63).
 __global__ void pvm_insert_kernel(uint32_t* __restrict__ words, uint32_t X, uint32_t Y, uint32_t Z, float side,
                                   const float* __restrict__ xyz, uint64_t n, int mode, int delta,
                                   uint32_t* __restrict__ outside) {
@@ -47,6 +50,8 @@ __global__ void pvm_insert_kernel(uint32_t* __restrict__ words, uint32_t X, uint
     const uint64_t i = i0 + lane;
     uint32_t word = 0xffffffffu;  // no word: at most 2^28 of them
     int byte = 0;
+    uint32_t old = 0u;
+    bool moves = false;  // the lane's own update would change the voxel
     if (i < n) {
       const uint32_t x = coord_to_voxel(__ldg(xyz + 3 * i), side), y = coord_to_voxel(__ldg(xyz + 3 * i + 1), side),
                      z = coord_to_voxel(__ldg(xyz + 3 * i + 2), side);
@@ -54,16 +59,19 @@ __global__ void pvm_insert_kernel(uint32_t* __restrict__ words, uint32_t X, uint
         const uint32_t id = (z * Y + y) * X + x;  // below 2^30
         word = id >> 2;
         byte = (int)(id & 3u);
+        old = *reinterpret_cast<volatile uint32_t*>(words + word);
+        const int cur = (int)(int8_t)(old >> (8 * byte));
+        moves = prob_steps(cur, mode, delta, 1) != cur;
       } else {
         out = true;
       }
     }
+    if (!__any_sync(0xffffffffu, moves)) continue;
     const unsigned same = __match_any_sync(0xffffffffu, word);
     const unsigned b0 = __ballot_sync(0xffffffffu, byte & 1), b1 = __ballot_sync(0xffffffffu, byte & 2);
     if (word != 0xffffffffu && __ffs(same) - 1 == lane) {
       const int times[4] = {__popc(same & ~b1 & ~b0), __popc(same & ~b1 & b0), __popc(same & b1 & ~b0), __popc(same & b1 & b0)};
       uint32_t* w = words + word;
-      uint32_t old = *reinterpret_cast<volatile uint32_t*>(w);
       for (;;) {  // ends: each retry follows another thread's successful swap
         uint32_t upd = 0u;
 #pragma unroll

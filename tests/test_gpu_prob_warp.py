@@ -25,3 +25,41 @@ def test_runs_of_points(n, spread):
         g.insertPointCloud(torch.as_tensor(pts), meaning)
         oracle.pvm_insert(o, dims, 1.0, pts, meaning)
         assert np.array_equal(g.data().cpu().numpy(), o)
+
+
+@pytest.mark.parametrize("meaning", [0, 1, 100, 129, 255])
+def test_settled_voxels_beside_moving_ones(meaning):
+    """Repeated inserts until every voxel of the cloud stands still, then the cloud with a few new voxels in it."""
+    dims = (37, 29, 23)
+    rng = np.random.default_rng(meaning)
+    g, o = gvx.ProbVoxelMap(dims, 1.0), oracle.pvm_empty(dims)
+    pts = (rng.random((20_000, 3)) * dims * [1, 1, 0.5]).astype(np.float32)
+    for k in range(16):
+        if k == 15:
+            pts[::97] += np.float32([0, 0, 11])
+        g.insertPointCloud(torch.as_tensor(pts), meaning)
+        oracle.pvm_insert(o, dims, 1.0, pts, meaning)
+        assert np.array_equal(g.data().cpu().numpy(), o)
+
+
+def test_settled_map_is_only_read():
+    """A cloud into a map that it no longer changes takes a third of the time it took when it did."""
+    m = gvx.ProbVoxelMap((256, 256, 256), 1.0)
+    pts = torch.rand(3_000_000, 3, device="cuda", generator=torch.Generator("cuda").manual_seed(0)) * 256
+
+    def insert_ms():
+        a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+        torch.cuda.synchronize()
+        a.record()
+        m.insertPointCloud(pts, 1)
+        b.record()
+        torch.cuda.synchronize()
+        return a.elapsed_time(b)
+
+    fresh = []
+    for _ in range(8):
+        m.clearMap()
+        fresh.append(insert_ms())
+    for _ in range(4):
+        m.insertPointCloud(pts, 1)
+    assert min(insert_ms() for _ in range(8)) < 0.45 * min(fresh)
