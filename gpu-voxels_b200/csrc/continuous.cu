@@ -308,7 +308,57 @@ MapView view(const gvx_dvm* m) {
                  (reinterpret_cast<uintptr_t>(m->d_vox) & 15u) == 0, num_voxels(m->dims)};
 }
 
+// Every integer up to 2^24, and the distance of an empty corner: roots whose bits
+// differ from sqrtf's, each value in both halves of the pair.
+__global__ void roots_check_kernel(unsigned long long* __restrict__ mismatches) {
+  constexpr int kLast = 1 << 24;
+  unsigned long long bad = 0;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i <= kLast + 1; i += gridDim.x * blockDim.x) {
+    const float v = (float)(i <= kLast ? i : kMaxObstacleDistance), w = (float)(kLast - min(i, kLast));
+    const float2 r = roots(make_float2(v, w));
+    bad += __float_as_uint(r.x) != __float_as_uint(sqrtf(v));
+    bad += __float_as_uint(r.y) != __float_as_uint(sqrtf(w));
+  }
+  if (bad) atomicAdd(mismatches, bad);
+}
+
+// 2^28 positions and sides from a counter: positions in and around a map, a few
+// ulp around every half of a side (where cells and rounding ties meet), float
+// positions, and any bits at all; sides of 1 mm to 1 m and any positive float.
+// Counts coordinates whose bits differ from the divide's; beyond 1e299 both have
+// to be as far, or no number.
+__global__ void lattice_check_kernel(unsigned long long* __restrict__ mismatches) {
+  unsigned long long bad = 0;
+  for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < (1ull << 28); i += (uint64_t)gridDim.x * blockDim.x) {
+    uint64_t h = (i + 1) * 0x9E3779B97F4A7C15ull;  // SplitMix64 (Steele, Lea, Flood, OOPSLA 2014)
+    h = (h ^ (h >> 30)) * 0xBF58476D1CE4E5B9ull;
+    h = (h ^ (h >> 27)) * 0x94D049BB133111EBull;
+    h ^= h >> 31;
+    const uint64_t g = h * 0xD6E8FEB86659FD93ull;
+    float side = __uint_as_float((uint32_t)(g >> 33) % 0x7F7FFFFFu + 1u);
+    if (i & 4) side = 0.001f + 0.999f * ((float)(g >> 40) * 0x1p-24f);
+    const double unit = (double)(h >> 11) * 0x1p-53;
+    double p = __longlong_as_double((long long)h);
+    if ((i & 3) == 1) p = (unit * 4096.0 - 1024.0) * (double)side;
+    if ((i & 3) == 2) p = __longlong_as_double(__double_as_longlong((double)((h >> 20) % 2050u) * 0.5 * (double)side) + (long long)(h & 7u) - 3);
+    if ((i & 3) == 3) p = (float)((unit * 2048.0 - 512.0) * (double)side);
+    const double got = lattice_coord(p, side, 1.0 / (double)side), want = p / (double)side - 0.5;
+    const bool same = __double_as_longlong(got) == __double_as_longlong(want) || (isnan(got) && isnan(want)) ||
+                      (fabs(got) > 1e299 && fabs(want) > 1e299 && signbit(got) == signbit(want));
+    bad += !same;
+  }
+  if (bad) atomicAdd(mismatches, bad);
+}
+
 }  // namespace
+
+cudaError_t check_query_arithmetic(unsigned long long* d_mismatches, cudaStream_t s) {
+  const cudaError_t e = cudaMemsetAsync(d_mismatches, 0, 2 * sizeof(unsigned long long), s);
+  if (e != cudaSuccess) return e;
+  roots_check_kernel<<<1024, 256, 0, s>>>(d_mismatches);
+  lattice_check_kernel<<<4096, 256, 0, s>>>(d_mismatches + 1);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_trilinear(const gvx_dvm* m, const float* d_xyz, uint64_t n, float* d_dist, float* d_grad, cudaStream_t s) {
   if (n == 0) return cudaSuccess;

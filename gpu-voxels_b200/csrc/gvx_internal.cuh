@@ -198,6 +198,8 @@ cudaError_t launch_meta_insert_self_coll(uint8_t* d_vox, gvx_dims d, float side,
 // Counts the quotients of the EDT bisector domain whose bits differ from the
 // IEEE divide (every numerator and divisor the sweeps can meet).
 cudaError_t check_bisector_quotient(unsigned long long* d_mismatches, cudaStream_t s);
+// d_mismatches: two counts, roots and lattice coordinates
+cudaError_t check_query_arithmetic(unsigned long long* d_mismatches, cudaStream_t s);
 // Resident warps of the fused batch launch (size of the batch stack pool).
 long long edt_batch_stack_warps();
 // Rows per staging chunk of the sweeps (16 or 32).

@@ -77,17 +77,26 @@ __device__ __forceinline__ void axis_setup(float p, float side, int n, int& i0, 
   }
 }
 
+// p / side - 0.5 in double, with inv = 1 / side rounded: the quotient is p * inv
+// with one residual correction (P. Markstein, IBM J. Res. Develop. 34(1), 1990)
+// in place of three FP64 divides per point.  It is the divide's: p * inv is within
+// 2 ulp of p / side, so the residual is exact in one fma (side has 24 significant
+// bits), and the second fma's exact value is off by 2^-51 ulp at most, where a
+// quotient by 24 bits lies 2^-25 ulp or more from a rounding midpoint.  An
+// infinity, and what is far beyond any map, stays as it is.
+// gvx_check_query_arithmetic compares it with the divide.
+__device__ __forceinline__ double lattice_coord(double p, float side, double inv) {
+  const double q0 = p * inv;
+  return (fabs(q0) < 1e300 ? fma(fma(-q0, (double)side, p), inv, q0) : q0) - 0.5;
+}
+
 // The same split of an FP64 position (sphere centres from the FP64 forward
 // kinematics): cell and fraction come from p / side - 0.5 in double, so only
 // the fraction (in [0, 1]) is rounded to float -- an FP32 position alone would
 // carry up to half an ulp of p (1.2e-5 voxel at 2.56 m with 1 cm voxels).
-// inv = 1 / side: the quotient is p * inv with one residual correction
-// (P. Markstein, IBM J. Res. Develop. 34(1), 1990) in place of three FP64
-// divides per point.
 __device__ __forceinline__ void axis_setup(double p, float side, double inv, int n, int& i0, int& i1, float& f,
                                            bool& free_axis) {
-  const double q0 = p * inv;
-  const double u = (fabs(q0) < 1e300 ? fma(fma(-q0, (double)side, p), inv, q0) : q0) - 0.5;  // an infinity stays one
+  const double u = lattice_coord(p, side, inv);
   const double hi = (double)(n - 1);
   free_axis = (u >= 0.0) && (u <= hi);
   const double uc = fmin(fmax(u, 0.0), hi);  // NaN -> 0
@@ -195,8 +204,8 @@ __device__ __forceinline__ float biased(uint32_t v) { return __uint_as_float(0x4
 // Roots of integers, rounded to nearest as sqrtf rounds them: an approximate
 // reciprocal root, one exact residual by fma and Markstein's correction
 // (P. Markstein, IBM J. Res. Develop. 34(1), 1990).  Bit for bit sqrtf on
-// every integer up to 2^24 and on kMaxObstacleDistance (all of them compared on a
-// B200).  2^-60 keeps the reciprocal finite at 0.
+// every integer up to 2^24 and on kMaxObstacleDistance, which
+// gvx_check_query_arithmetic compares.  2^-60 keeps the reciprocal finite at 0.
 __device__ __forceinline__ float2 roots(float2 v) {
   const float2 w = __fadd2_rn(v, both(0x1p-60f));
   float2 y;

@@ -137,6 +137,11 @@ GVX_API gvx_status gvx_dvm_edt_check(gvx_dvm *m, uint32_t *flags);
  * IEEE divide for every numerator (|num| < 2^21) and divisor (even, 2..2046)
  * the sweeps can meet; *mismatches = 0 when all agree.  Synchronous. */
 GVX_API gvx_status gvx_check_bisector_quotient(uint64_t *mismatches);
+/* Self-check of the arm kernels' arithmetic on this device: their roots against
+ * sqrtf for every integer up to 2^24 and MAX_OBSTACLE_DISTANCE, and their FP64
+ * lattice coordinates p / side - 0.5 against the IEEE divide for 2^28 positions
+ * and sides.  The counts of results whose bits differ.  Synchronous. */
+GVX_API gvx_status gvx_check_query_arithmetic(uint64_t *roots, uint64_t *coordinates);
 
 /* No counterpart in the reference.  The same EDT as gvx_dvm_edt, in place on
  * caller-owned device voxels (uint32 DistanceVoxels, x fastest, 16-byte

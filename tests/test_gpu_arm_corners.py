@@ -2,12 +2,15 @@
 site word (near, far, empty, one field of 1023, bits above the fields), spheres
 in and outside the map, at every position of an aligned 16-byte word, in the
 map's last words and on one-voxel axes."""
+import ctypes
+
 import numpy as np
 import pytest
 import torch
 
 import gvx
 import oracle
+from gvx import _abi
 
 pytestmark = pytest.mark.gpu
 
@@ -24,6 +27,14 @@ def _words(rng, n, odd):
         v = np.where(kind == 4, v | 0x40000000, v)
         v = np.where(kind == 5, v & 0x3FF003FF | 1022 << 10, v)
     return v.astype(np.uint32)
+
+
+def test_roots_and_lattice_coordinates_equal_the_general_forms():
+    """Every root the arm kernels can take is sqrtf's, and their position divided by the side is the IEEE divide's, ties
+    and cell faces included."""
+    roots, coordinates = ctypes.c_uint64(1), ctypes.c_uint64(1)
+    _abi.call("gvx_check_query_arithmetic", ctypes.byref(roots), ctypes.byref(coordinates))
+    assert (roots.value, coordinates.value) == (0, 0)
 
 
 @pytest.mark.parametrize("odd", [False, True])
