@@ -763,7 +763,7 @@ def main():
 
     dvm.clearMap()
     dvm.insertPointCloud(pts)
-    edt_config = dvm.autotune()  # untimed: picks the sweep configuration for this map
+    edt_config = dvm.autotune()  # untimed: the sweeps' configuration (sweeps_ms below; the headline map is the row search's)
     clocks = ClockSampler(local).start()
     for _ in range(args.warmup):
         step()

@@ -298,9 +298,9 @@ __global__ void __launch_bounds__(256) lists_collide_bits_kernel(const uint32_t*
   }
   // Entry e of lane l in group g is g * kG + e * 32 + l: each load covers 32
   // consecutive entries of a sorted list, so its bit lookups fall in few lines.
-  // The loop is bound by instruction issue: entries are counted down in 32
-  // bits from the warp's first one, a whole group is loaded without a check per
-  // entry, and one vote tells whether any of its 128 entries is a candidate
+  // The loop is bound by instruction issue: the lane's entries left are counted
+  // down, a whole group is loaded without a check per entry, and one vote tells
+  // whether any of its 128 entries is a candidate
   // (37 instructions per 32 entries before, most of them 64-bit index checks).
   const uint32_t in_map = (uint32_t)min(map_n, (uint64_t)0xFFFFFFFFu);
   const uint32_t* idp = ids + g_begin * kG + lane;

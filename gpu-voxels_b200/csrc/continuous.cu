@@ -74,7 +74,8 @@ constexpr int kThreads = kWarpsPerBlock * 32;
 constexpr int kMaxBlockConfigs = 64;
 // Blocks of an SM the clearance and cost kernels keep room for: four (64
 // registers) take 512 trajectories at once, where three (75 to 80 registers)
-// left a second wave (cost 52 us against 50, 4096 clearances 11.9 against 10.3).
+// left a second wave (cost 52 us against 50, 4096 clearances 11.9 against 10.3),
+// though at 64 they spill 36 and 12 bytes a thread.
 // The adjoint's FP64 sums spill at 64 and at 80 registers (91 us); left at 124 it takes 74.
 constexpr int kArmBlocks = 4;
 

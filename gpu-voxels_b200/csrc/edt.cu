@@ -7,9 +7,10 @@
 //
 // Maps whose sites all lie in their own voxels (after insertPointCloud, or
 // voxelize_edt's occupancy bits) and whose rows and columns have at most 512
-// voxels go to the row search (edt_search.cu).  The sweeps below take the
-// others: longer axes, maps transformed before or written by the caller, the
-// workspace built into the library, and the single-stage entry point.
+// voxels go to the row search (edt_search.cu), unless they are a batch of many
+// small ones or too large for it in the workspace built into the library.  The
+// sweeps below take the others: longer axes, maps transformed before or written by
+// the caller, such batches, and the single-stage entry point.
 //
 // Three sweeps (pass Z one launch, passes Y and X one fused launch):
 //   pass Z : phase 1 (kernelPBAphase1FloodZ, VoxelMapOperationsPBA.hpp:63-124)

@@ -31,14 +31,14 @@
 // (512^3 depth scene); with lanes along x, as the sweeps have them, it was up to
 // 7.9 times.
 //
-// What bounds it: instruction issue and the 2-cycle integer pipe (65 % and 70 %
-// busy; a candidate costs one add-and-min, no divide, no per-lane control
-// flow); DRAM is a third busy.  Measured on a B200 against the sweeps of edt.cu
-// (whole calls, warm): 512^3 depth scene 798 us against 1710 (pass Y 344, pass X
-// 426); 128^3 with 50k box points 36 against 183 (the sweeps walk 128 rows one
-// after another per pass, here 8 warps share a column); 203 x 331 x 157 in three
-// calls 139 against 491; 24 uneven maps of 64 to 384 per axis in one batch 1499
-// against 2606.
+// What bounds it: instruction issue (67 % of the cycles in pass Y, 60 % in pass X;
+// 352^3 depth scene) and the 2-cycle integer pipe (60 % and 57 %; a candidate
+// costs one add-and-min, no divide, no per-lane control flow); DRAM is a third
+// busy.  Measured on a B200 against the sweeps of edt.cu (whole calls, warm): 512^3
+// depth scene 790 us against 1710 (pass Y 345, pass X 429); 128^3 with 50k box
+// points 36 against 183 (the sweeps walk 128 rows one after another per pass, here
+// 8 warps share a column); 203 x 331 x 157 in three calls 139 against 491; 24 uneven
+// maps of 64 to 384 per axis in one batch 1505 against 2606.
 //
 // The searching loops are kept rolled: unrolled over a warp's rows the code
 // outgrew the instruction caches (at 352^3 the largest stall was 'no
@@ -88,9 +88,7 @@ __host__ __device__ __forceinline__ int seg_rows(int L) { return 16 * ((L + 127)
 // candidates (16 bits); then `extra` words.  At 512 rows a third of an SM's
 // shared memory to the byte.
 __host__ __device__ __forceinline__ int key_rows(int L) { return (L + 3) & ~3; }
-__host__ __device__ __forceinline__ int weight_words(int L) {
-  return 2 * kWarps * seg_rows(L) + (seg_rows(L) < 64 ? 72 : 0);  // short segments look past their end
-}
+__host__ __device__ __forceinline__ int weight_words(int L) { return 2 * kWarps * seg_rows(L); }
 __host__ __device__ __forceinline__ int least_words(int L) { return kWarps * seg_rows(L); }
 __host__ __device__ __forceinline__ int search_smem_words(int L, int extra) {
   return key_rows(L) * 32 + weight_words(L) + kWarps * 32 + least_words(L) + extra;
@@ -312,8 +310,7 @@ __device__ __forceinline__ void segment_starts(const Search& s, int warp, int S,
 // (called by all threads; synchronises).  out.begin(none) tells whether the
 // lane's column has no site; then the warp's rows come in ascending groups:
 // out.rows(r, k, same) has the least keys of rows r .. r + 7 (same: one site
-// for all eight in every column), out.same16(r, k, d2) the key of row r of the
-// site that rows r .. r + 15 share (shift_key's d2); then out.finish().
+// for all eight in every column); then out.finish().
 template <class Out>
 __device__ __forceinline__ void search_rows(const Search& s, Out& out) {
   const int S = seg_rows(s.L);
@@ -503,8 +500,7 @@ __device__ __forceinline__ float sqrt_approx(float v) {
 // square root gives to 2^-12.  A site's word is made once where several rows
 // share it.  The words go out 8 x (a 32-byte sector) per z, 16 z at a time
 // through 512 bytes per warp: whole sectors with 16-byte stores where the map's
-// rows are aligned (vec), else word by word; 16 rows of one site go out 16 x
-// per z straight from the lanes.
+// rows are aligned (vec), else word by word.
 struct OutX {
   const uint32_t* src;  // row 0 of this lane's column in `field`
   uint32_t* stage;
@@ -631,8 +627,8 @@ __device__ __forceinline__ void item_x(uint32_t* smem, const uint32_t* field, ui
 
 // Resident blocks the registers must allow: pass Y four (64 registers; four fit
 // the shared memory up to 384 rows, and 69 registers took three, 24 maps' pass
-// Y 682 us against 634), pass X three (at 64 registers it spills: 512^3 447 ->
-// 486 us).
+// Y 682 us against 634, though the batch form spills 16 bytes at 64), pass X three
+// (at 64 registers it spills more: 512^3 447 -> 486 us).
 constexpr int kStageWords = kWarps * 128;
 int smem_y(int Y) { return search_smem_words(Y, 2 * Y) * 4; }
 int smem_x(int X) { return search_smem_words(X, kStageWords) * 4; }

@@ -19,7 +19,9 @@
 // every device context the process creates.  Either way it stays there until
 // the process exits.  Maps whose EDT workspace would exceed it (more than
 // 16,777,216 voxels once x and y are rounded up to multiples of 32; 256^3
-// fits) are rejected with GVX_ERR_OUT_OF_DOMAIN.
+// fits) are rejected with GVX_ERR_OUT_OF_DOMAIN.  The row search runs in it up to
+// 493,504 columns of 32 z (15,792,128 voxels where Z is a multiple of 32); the maps
+// between the two limits are swept.
 //
 // The fused y -> x sweep's bounded waits report a give-up in an error word
 // inside this workspace (word dims.z + 1, zeroed by every call), which

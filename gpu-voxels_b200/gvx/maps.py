@@ -148,7 +148,7 @@ class DistanceVoxelMap:
 
     def edt_pass(self, pass_index: int) -> None:
         """One EDT stage: 0 = z sweep, 1 = y sweep, 2 = x sweep, 3 = y and x
-        sweeps as the one fused launch parallelBanding3D uses."""
+        sweeps as one fused launch (parallelBanding3D's where it sweeps)."""
         call("gvx_dvm_edt_pass", self._h, int(pass_index), _stream())
 
     def autotune(self, force: bool = False) -> dict:

@@ -109,8 +109,9 @@ GVX_API gvx_status gvx_dvm_edt_pass(gvx_dvm *m, int pass, gvx_stream stream);
 /* EDT launch configuration chosen by the autotuner: rows per staging chunk of
  * the sweeps (16 or 32; 0 = library default), whether the y and x sweeps run
  * as one fused launch (1) or two (0), and the time measured for it.  The sweeps
- * run for maps longer than 512 in x or y and for maps holding sites outside
- * their own voxels; the other maps' EDT (a search per row) has no setting. */
+ * run for maps longer than 512 in x or y, for maps holding sites outside their
+ * own voxels and for batches of many small maps; the other maps' EDT (a search
+ * per row) has no setting. */
 typedef struct {
   uint32_t rows;
   uint32_t fused;
